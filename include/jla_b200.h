@@ -205,6 +205,14 @@ int jla_ssd_layer_bwd(int dtype, int64_t tokens, int H, int P, const void* x, co
                       const float* d, const void* dv, const float* dg, const void* dy, void* dx, float* ddt, float* da,
                       float* dd, jla_stream_t stream);
 
+/* One decoding step of a Mamba-2 layer's scan, the three glue steps above and the scan itself in one pass over the
+ * state: `p` is the simple_gla problem with T = 1, q = C, k = B, v = x (all 16-bit), scale, h0; its g is not read.
+ *   v = round(x * dt), g = dt * A, o = the scan's output, y = round(o) (D NULL) or round(round(o) + D * x)
+ * K in (64, 128, 256), V a multiple of 64. final_state may be NULL. Replaces one token of mamba2_ssd
+ * (src/jla/layers/ssm.py:183-230). */
+int jla_ssd_step(const jla_problem* p, const float* dt, const float* a, const float* d, void* y, float* final_state,
+                 jla_stream_t stream);
+
 /* Gate activations in front of the kernels, forward and backward in one pass each; replaces the XLA fusions of
  * _mamba_gate and _write_strength in the Gated DeltaNet and KDA mixers (src/jla/layers/linear_attention.py:84-86,
  * 159-162, 295-297, 324-328):

@@ -63,6 +63,7 @@ const char* shape_problem(const jla_problem& p) {
 
 const char* unsupported(const jla_problem& p) {
   if (const char* why = shape_problem(p)) return why;
+  if (token_step_applies(p)) return nullptr;
   return resolve_path(p) == JLA_PATH_RECURRENT ? recurrent_unsupported(p) : chunked_unsupported(p);
 }
 
@@ -126,7 +127,7 @@ size_t jla_residual_bytes(const jla_problem* p) {
 }
 
 size_t jla_fwd_scratch_bytes(const jla_problem* p) {
-  if (!p || unsupported(*p)) return 0;
+  if (!p || unsupported(*p) || token_step_applies(*p)) return 0;
   return resolve_path(*p) == JLA_PATH_RECURRENT ? 0 : chunked_fwd_scratch_bytes(*p);
 }
 
@@ -143,6 +144,7 @@ int jla_linear_attention_fwd(const jla_problem* p, const jla_fwd_io* io, jla_str
     return JLA_ERR_BAD_ARGUMENT;
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  if (token_step_applies(*p)) return token_step_fwd(*p, *io, s);
   return resolve_path(*p) == JLA_PATH_RECURRENT ? recurrent_fwd(*p, *io, s) : chunked_fwd(*p, *io, s);
 }
 

@@ -150,6 +150,8 @@ struct Carver {
 int recurrent_fwd(const jla_problem& p, const jla_fwd_io& io, cudaStream_t stream);
 int recurrent_bwd(const jla_problem& p, const jla_bwd_io& io, cudaStream_t stream);
 size_t recurrent_bwd_scratch_bytes(const jla_problem& p);
+bool token_step_applies(const jla_problem& p);  // token_step.cu
+int token_step_fwd(const jla_problem& p, const jla_fwd_io& io, cudaStream_t stream);
 
 // dq/dk epilogue shared by both paths: sums per-value-head fp32 gradients over each key group, applies the
 // L2-norm backward when the op normalised q/k itself, rounds to the tensor dtype.

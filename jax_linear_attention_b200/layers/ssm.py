@@ -36,6 +36,12 @@ def mamba2_ssd(x, dt, a, b, c, *, d=None, segment_ids=None, initial_state=None, 
         raise ValueError(f"b, c must be [B, T, G, N] with H % G == 0; got {tuple(b.shape)}, {tuple(c.shape)}")
     if a.shape != (heads,):
         raise ValueError(f"a must be [H] = {(heads,)}; got {tuple(a.shape)}")
+    if (x.shape[1] == 1 and x.is_cuda and x.dtype in _DTYPES and impl in ("auto", "cuda")
+            and not (torch.is_grad_enabled() and any(t is not None and t.requires_grad
+                                                     for t in (x, dt, a, b, c, d, initial_state)))):
+        out = _step(x, dt, a, b, c, d, segment_ids, initial_state, output_final_state, chunk_size, precision)
+        if out is not None:
+            return out
     fused = x.is_cuda and x.dtype in (torch.bfloat16, torch.float16) and x.shape[3] % 8 == 0
     # the output side's backward leaves dy here for the input side's backward (which runs after it: v and g lie
     # between them), so that dx = dv * dt + D * dy, ddt, dA and dD come from one pass over x, dv and dy
@@ -60,6 +66,32 @@ def mamba2_ssd(x, dt, a, b, c, *, d=None, segment_ids=None, initial_state=None, 
         else:
             y = (y.float() + d.float()[:, None] * x.float()).to(y.dtype)
     return y, state
+
+
+def _step(x, dt, a, b, c, d, segment_ids, initial_state, output_final_state, chunk_size, precision):
+    """One decoding step as one kernel (``jla_ssd_step``), or None where the general form has to run or to complain."""
+    batch, _, heads, width = x.shape
+    groups, n = b.shape[2:]
+    options = dict(initial_state=initial_state, segment_ids=segment_ids, chunk_size=chunk_size, precision=precision)
+    if (c.dtype != x.dtype or n not in (64, 128, 256) or width % 64 or precision == "chunked"
+            or (d is not None and d.shape != (heads,))
+            or ops.cuda.unsupported_reason("simple_gla", c, b.to(c.dtype), x, (dt,), options) is not None):
+        return None
+    p = ops.cuda._problem("simple_gla", x.dtype, batch, 1, heads, groups, n, width, 0, 1.0, 0, precision)
+    dev = x.device
+    keep = [t if t is None else t.to(device=dev, dtype=td).contiguous() for t, td in
+            ((c, c.dtype), (b, c.dtype), (x, x.dtype), (initial_state, torch.float32), (dt, torch.float32),
+             (a, torch.float32), (d, torch.float32))]
+    p.q, p.k, p.v, p.h0, dt_ptr, a_ptr, d_ptr = (None if t is None else t.data_ptr() for t in keep)
+    y = torch.empty_like(keep[2])
+    final = torch.empty(batch, heads, n, width, dtype=torch.float32, device=dev) if output_final_state else None
+    stream = torch.cuda.current_stream(dev).cuda_stream
+    with torch.cuda.device(dev):
+        _lib.check(_lib.load().jla_ssd_step(C.byref(p), C.c_void_p(dt_ptr), C.c_void_p(a_ptr), C.c_void_p(d_ptr),
+                                            C.c_void_p(y.data_ptr()),
+                                            C.c_void_p(None if final is None else final.data_ptr()),
+                                            C.c_void_p(stream)), "ssd step")
+    return y, final
 
 
 def _glue_call(name: str, x: torch.Tensor, *args):

@@ -127,7 +127,7 @@ def unsupported_reason(kind: str, q, k, v, gates: tuple, options: dict, *, read_
         return str(err)
     blocks = _value_blocks(kind, q.dtype, key_dim, value_dim, precision, read_key)  # wide value heads run in blocks
     p = _problem(kind, q.dtype, batch, seq_len, heads * blocks, kv_heads, key_dim, value_dim // blocks,
-                 0 if cu is None else max(rows, 0), 1.0, 0, precision)
+                 0 if cu is None else max(rows, 0), 1.0, _lib.FLAG_SAVE_RESIDUALS, precision)  # (a call with gradients)
     if read_key:
         p.k_read = 1  # only looked at for being non-NULL
     return _lib.unsupported_reason(p)
@@ -210,7 +210,7 @@ class _LinearAttention(torch.autograd.Function):
         o = torch.empty_like(v)
         final = torch.empty(rows, H, K, V, dtype=torch.float32, device=dev) if cfg["output_final_state"] else None
         res_bytes = lib.jla_residual_bytes(C.byref(p)) if needs_grad else 0
-        share = _PassOptions.share
+        share = _PassOptions.share if T > 1 else None  # (a single token has no tables to share)
         if share is not None:  # one residual-layout buffer for a run of calls; the first one fills its tables
             # identity and version of the tensors the CALLER passed (not of the float32 / int32 / contiguous copies
             # made on the way here, whose addresses can be reused by the allocator inside one shared_prep block)
@@ -334,6 +334,12 @@ def _split_applies(kind, q, v, cu_seqlens, initial_state, precision) -> int:
     return pieces(1, v.shape[2], q.shape[1], delta=kind != "simple_gla", sm_count=sms)
 
 
+def _is_step(q, k, v, g, beta, initial_state, cu_seqlens, precision) -> bool:
+    """A decoding step (one token per row and nothing to differentiate), which ``csrc/token_step.cu`` runs."""
+    return (q.shape[1] == 1 and cu_seqlens is None and _path(precision) != "chunked"
+            and not any(x is not None and x.requires_grad for x in (q, k, v, g, beta, initial_state)))
+
+
 def _run_value_blocks(n, kind, q, k, v, g, beta, *, initial_state, output_final_state, **options):
     """The call with every value head cut into ``n`` heads of 128 channels (see ``_value_blocks``): ``v`` and ``o``
     are views, the gates are repeated per block (autograd sums their gradients back), the states are permuted."""
@@ -373,6 +379,8 @@ def _run(kind: str, q, k, v, g, beta, *, scale, initial_state, output_final_stat
     if scale is None:
         scale = q.shape[-1] ** -0.5
     blocks = _value_blocks(kind, q.dtype, q.shape[-1], v.shape[-1], _path(precision), k_read is not None)
+    if blocks > 1 and _is_step(q, k, v, g, beta, initial_state, cu_seqlens, precision):
+        blocks = 1  # the decoding-step kernel takes wide value heads as they are
     if blocks > 1:
         return _run_value_blocks(blocks, kind, q, k, v, g, beta, scale=scale, initial_state=initial_state,
                                  output_final_state=output_final_state, cu_seqlens=cu_seqlens, segment_ids=segment_ids,
