@@ -4,13 +4,24 @@
 // reset, decay, delta write, read; with cu_seqlens every sequence is a row with its own initial and
 // final state (reference.py:170-203). Arithmetic is fp32 FMA on CUDA cores whatever the storage dtype,
 // so this path serves the fp32 configuration (relative L2 error <= 1e-5 against the fp32 reference) and
-// is the on-device cross-check of the tensor-core kernels. It is latency-bound by design: one CTA per
-// (row, head), the K x V state distributed over the CTA's registers.
+// is the on-device cross-check of the tensor-core kernels.
 //
-// Thread layout: thread = (ks, v) with v the value column and ks one of KS = K / KPT key slices; a thread
-// owns state entries S[ks*KPT .. ks*KPT+KPT-1][v]. Reductions over keys go through shared memory (KS
-// partials per column); reductions over value columns use warp shuffles (V is a power of two).
+// The walks are bound by latency: one token's chain is decay -> key dot product -> write, and it repeats for every
+// token of a row. So a walk does nothing but its chain. The columns of the state are independent recurrences: a warp
+// owns 32 / KL columns with the key channels over KL lanes (16 channels a thread), so the key reduction is log2(KL)
+// shuffles and no barrier; a CTA of four warps stages eight tokens at a time in shared memory, the next eight already on
+// their way to registers. The backward has two such walks that need nothing of each other and run side by side in one
+// launch: the forward state with a checkpoint every TB tokens, and the state gradient, which never reads the state
+// (dS_t = decay (dS_{t+1} + ...), du_t = k_t dS), with its own checkpoints. Everything that needs both, the gradients
+// of q, k and the gates, is then computed for all blocks of TB tokens at once from the two checkpoints of a block.
+//
+// fp32 B1 T512 H4 K = V = 64 forward + backward: 122 + 146 + 17 us of kernels (walk, two walks, block gradients); the
+// one-CTA-per-head scan with barriers in every token and the gradient reductions inside the walk took 410 + 2718 us.
+// A token of a walk is 108 instructions of one warp, 240 ns: its chain and the waits of a warp that is alone on its
+// scheduler.
 #include <stdio.h>
+
+#include <type_traits>
 
 #include "common.cuh"
 #include "profile.cuh"
@@ -18,7 +29,14 @@
 namespace jla {
 namespace {
 
-constexpr int TB = 16;  // tokens staged in shared memory per block
+constexpr int TB = 16;        // tokens between two checkpoints = tokens of a block of block_grads_kernel
+constexpr int SB = 8;         // tokens that a walk stages at a time
+constexpr int NW = 4;         // warps of a walk's CTA
+constexpr int KPT = 16;       // key channels of a thread in the walks
+constexpr int GT = 256;       // threads of block_grads_kernel
+constexpr int CT = 64;        // its channel tile
+constexpr int VT = 32;        // its tile of value columns
+constexpr int VTS = VT + 4;   // (stride of a staged state row: 16-byte reads of 8 neighbouring rows hit 8 bank groups)
 
 struct RecParams {
   Rows rows;
@@ -37,356 +55,683 @@ struct RecParams {
   float* dkr_acc;          // [B*T, H, K] f32: gradient of k_read (with k_read only)
   void* dv;
   float *dg, *dbeta, *dh0;
-  float* ckpt;  // [H][total_blocks][K*V]
-  float* spre;  // [rows*H][TB][K*V]
-  long total_blocks;
+  // [H][slots][K*V]: the state entering every block of a row and the one leaving its last block; the state gradient
+  // coming from behind every block. Slot of block b of a row: slot0(row) + b (slots of a row: its blocks + 1).
+  float *s_ckpt, *ds_ckpt;
+  float *resid, *du;  // [B*T, H, V] f32: v_t - r_t and the gradient of the written value u_t
+  int* slot_row;      // [slots]: the row of a slot (unwritten slots hold anything: the reader checks)
+  long slots;
+
+  __device__ __forceinline__ long slot0(int r, int tok0) const { return tok0 / TB + 2L * r; }
 };
 
-struct Smem {
-  float *qs, *ks, *kr, *vs, *eg, *bs, *inv, *part, *dos, *us, *es, *red;  // kr: the read key (= ks without k_read)
-  int* rs;
+template <int KL>
+__device__ __forceinline__ float key_sum(float x) {  // over the KL neighbouring lanes of a column
+#pragma unroll
+  for (int off = KL / 2; off > 0; off >>= 1) x += __shfl_xor_sync(0xffffffffu, x, off);
+  return x;
+}
+
+__device__ __forceinline__ float warp_sum(float x) { return key_sum<32>(x); }
+__device__ __forceinline__ double warp_sum(double x) {
+#pragma unroll
+  for (int off = 16; off > 0; off >>= 1) x += __shfl_xor_sync(0xffffffffu, x, off);
+  return x;
+}
+
+// ---- staging of the walks --------------------------------------------------------------------------
+template <int KL>
+struct WalkSmem {
+  static constexpr int KP = KL * KPT;        // channels, padded with zeros
+  static constexpr int NC = NW * (32 / KL);  // value columns of the CTA
+  float q[SB][KP], k[SB][KP], kr[SB][KP], e[SB][KP];
+  float x[SB][NC];  // v, or the upstream gradient
+  float es[SB], bs[SB];
+  int rs[SB], any_reset;
 };
 
-__host__ __device__ inline size_t smem_floats(int K, int V, int KS, bool bwd) {
-  size_t n = 3 * TB * K + TB * V + TB * K + TB + 2 * TB + TB /*rs*/ + 3 * (size_t)KS * V;
-  if (bwd) n += 3 * TB * V + 2 * (size_t)(4 * 8 * K + 64);
-  return n;
+// One batch of SB tokens on its way from global memory to shared memory. Warp w carries tokens w and w + NW whole, so
+// the L2 norm of q and k (reference.py:128-129) is a warp reduction. Tokens behind the end of the row are staged as
+// tokens that change nothing (zero vectors, decay 1).
+template <typename T, int KL>
+struct Stage {
+  static constexpr int M = KL / 2 > 0 ? KL / 2 : 1;            // channels of a lane
+  static constexpr int NC = WalkSmem<KL>::NC;
+  static constexpr int NX = SB * NC / (NW * 32) > 0 ? SB * NC / (NW * 32) : 1;
+  T q[SB / NW][M], k[SB / NW][M], kr[SB / NW][M], x[NX];
+  float g[SB / NW][M], gs, beta;
+  int seg_reset;
+
+  __device__ __forceinline__ void load(const RecParams& p, const T* xs, bool want_q, int tok, int nb, int row_tok0, int h,
+                                       int hk, int v0) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int n = 0; n < SB / NW; ++n) {
+      const int j = warp + n * NW;
+      const long key = ((long)(tok + j) * p.Hk + hk) * p.K, val = ((long)(tok + j) * p.H + h) * p.K;
+#pragma unroll
+      for (int m = 0; m < M; ++m) {
+        const int c = lane + 32 * m;
+        const bool ok = j < nb && c < p.K;
+        q[n][m] = ok && want_q ? static_cast<const T*>(p.q)[key + c] : from_f32<T>(0.f);
+        k[n][m] = ok ? static_cast<const T*>(p.k)[key + c] : from_f32<T>(0.f);
+        if (p.k_read) kr[n][m] = ok ? static_cast<const T*>(p.k_read)[val + c] : from_f32<T>(0.f);
+        if (p.gate == 2) g[n][m] = ok ? p.g[val + c] : 0.f;
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < NX; ++m) {
+      const int idx = threadIdx.x + m * NW * 32, j = idx / NC, c = idx - j * NC;
+      x[m] = j < nb && v0 + c < p.V ? xs[((long)(tok + j) * p.H + h) * p.V + v0 + c] : from_f32<T>(0.f);
+    }
+    gs = 0.f, beta = 0.f, seg_reset = 0;
+    if (threadIdx.x < nb) {
+      const long t = (long)(tok + threadIdx.x) * p.H + h;
+      if (p.gate == 1) gs = p.g[t];
+      beta = p.delta ? p.beta[t] : 1.f;
+      seg_reset = p.rows.resets(tok + threadIdx.x, row_tok0) ? 1 : 0;
+    }
+  }
+
+  __device__ __forceinline__ void commit(const RecParams& p, WalkSmem<KL>& s, bool want_q, int nb) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int n = 0; n < SB / NW; ++n) {
+      const int j = warp + n * NW;
+      float qf[M], kf[M];
+      float sq = 0.f, sk = 0.f;
+#pragma unroll
+      for (int m = 0; m < M; ++m) {
+        qf[m] = to_f32(q[n][m]), kf[m] = to_f32(k[n][m]);
+        sq += qf[m] * qf[m], sk += kf[m] * kf[m];
+      }
+      if (p.l2norm) {  // the reference rounds the normalised tensors to the input dtype (reference.py:69)
+        const float iq = rsqrtf(warp_sum(sq) + 1e-6f), ik = rsqrtf(warp_sum(sk) + 1e-6f);
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+          qf[m] = to_f32(from_f32<T>(qf[m] * iq));
+          kf[m] = to_f32(from_f32<T>(kf[m] * ik));
+        }
+      }
+#pragma unroll
+      for (int m = 0; m < M; ++m) {
+        const int c = lane + 32 * m;
+        if (c >= WalkSmem<KL>::KP) break;
+        if (want_q) s.q[j][c] = qf[m];
+        s.k[j][c] = kf[m];
+        if (p.k_read) s.kr[j][c] = to_f32(kr[n][m]);
+        if (p.gate == 2) s.e[j][c] = expf(g[n][m]);
+      }
+    }
+#pragma unroll
+    for (int m = 0; m < NX; ++m) {
+      const int idx = threadIdx.x + m * NW * 32;
+      if (idx < SB * NC) s.x[idx / NC][idx % NC] = to_f32(x[m]);
+    }
+    if (threadIdx.x < 32) {
+      const unsigned any = __ballot_sync(0xffffffffu, seg_reset);
+      if (threadIdx.x < SB) {
+        s.es[threadIdx.x] = p.gate == 1 && threadIdx.x < nb ? expf(gs) : 1.f;
+        s.bs[threadIdx.x] = beta;
+        s.rs[threadIdx.x] = seg_reset;
+      }
+      if (threadIdx.x == 0) s.any_reset = any != 0;
+    }
+  }
+};
+
+// Two channels in one 64-bit register pair: sm_100's packed fp32 instructions, each half rounded like the scalar one.
+// The walks issue half the arithmetic instructions this way, which is what is left of a token next to its chain.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2f(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2f(f32x2 x) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(x));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
 }
 
-__device__ inline Smem carve(float* base, int K, int V, int KS, bool bwd) {
-  Smem s;
-  s.qs = base;
-  s.ks = s.qs + TB * K;
-  s.kr = s.ks + TB * K;
-  s.vs = s.kr + TB * K;
-  s.eg = s.vs + TB * V;
-  s.bs = s.eg + TB * K;
-  s.inv = s.bs + TB;
-  s.rs = reinterpret_cast<int*>(s.inv + 2 * TB);
-  s.part = reinterpret_cast<float*>(s.rs + TB);
-  s.dos = s.part + 3 * KS * V;
-  s.us = s.dos + TB * V;
-  s.es = s.us + TB * V;
-  s.red = s.es + TB * V;
-  return s;
+constexpr int KP2 = KPT / 2;
+typedef f32x2 Chan[KP2];  // the channels of a thread
+
+__device__ __forceinline__ float dot(const Chan& a, const Chan& b) {
+  f32x2 s[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) s[i] = mul2(a[i], b[i]);
+#pragma unroll
+  for (int i = 4; i < KP2; ++i) s[i & 3] = fma2(a[i], b[i], s[i & 3]);
+  const float2 x = unpack2f(add2(add2(s[0], s[1]), add2(s[2], s[3])));
+  return x.x + x.y;
+}
+__device__ __forceinline__ void axpy(Chan& S, const Chan& a, float u) {
+  const f32x2 uu = pack2f(u, u);
+#pragma unroll
+  for (int i = 0; i < KP2; ++i) S[i] = fma2(a[i], uu, S[i]);
+}
+__device__ __forceinline__ void scale_by(Chan& S, float e) {
+  const f32x2 ee = pack2f(e, e);
+#pragma unroll
+  for (int i = 0; i < KP2; ++i) S[i] = mul2(S[i], ee);
+}
+__device__ __forceinline__ void scale_by(Chan& S, const Chan& e) {
+#pragma unroll
+  for (int i = 0; i < KP2; ++i) S[i] = mul2(S[i], e[i]);
+}
+__device__ __forceinline__ void clear(Chan& S) {
+#pragma unroll
+  for (int i = 0; i < KP2; ++i) S[i] = 0;
 }
 
-// Stage `nb` tokens starting at flat token `tok` into shared memory as fp32 (q, k of key head hk; v, gates
-// of head h), including the in-op L2 norm of q and k (reference.py:128-129) and the per-token reset flags.
+// A thread's place in a walk: key lane kl of column v; channel of its entry i (16-byte shared-memory reads of the KL
+// lanes are neighbours).
+template <int KL>
+struct Lane {
+  int kl, col, v;
+  bool active;
+  __device__ __forceinline__ Lane(int v0, int V) {
+    const int lane = threadIdx.x & 31;
+    kl = lane % KL;
+    col = (threadIdx.x >> 5) * (32 / KL) + lane / KL;
+    v = v0 + col;
+    active = v < V;
+  }
+  __device__ __forceinline__ int channel(int i) const { return (i >> 2) * (4 * KL) + kl * 4 + (i & 3); }
+  __device__ __forceinline__ void read(const float* src, Chan& dst) const {
+#pragma unroll
+    for (int i = 0; i < KPT; i += 4) {
+      const ulonglong2 x = *reinterpret_cast<const ulonglong2*>(src + channel(i));
+      dst[i / 2] = x.x, dst[i / 2 + 1] = x.y;
+    }
+  }
+  __device__ __forceinline__ void load_state(const float* src, int K, int V, Chan& S) const {
+#pragma unroll
+    for (int i = 0; i < KPT; i += 2) {
+      const bool ok = src && active && channel(i) < K;  // (K is even)
+      const float* at = src + (long)channel(i) * V + v;
+      S[i / 2] = ok ? pack2f(at[0], at[V]) : 0;
+    }
+  }
+  __device__ __forceinline__ void store_state(float* dst, int K, int V, const Chan& S) const {
+#pragma unroll
+    for (int i = 0; i < KPT; i += 2) {
+      if (!active || channel(i) >= K) continue;
+      float* at = dst + (long)channel(i) * V + v;
+      const float2 x = unpack2f(S[i / 2]);
+      at[0] = x.x, at[V] = x.y;
+    }
+  }
+};
+
+// What a walk does per token, fixed at compile time so that the eight staged tokens are one straight line of code (the
+// key vectors of a token are then read while the token before it waits for its shuffles; with run-time branches in the
+// token body the fp32 walk of K = V = 64 took 326 ns a token).
+enum { kHeadDecay = 0, kHeadDelta = 1, kChannelDelta = 2 };  // scalar (or no) gate; with the delta rule; per key channel
+template <int MODE>
+struct Walk {
+  static constexpr bool delta = MODE != kHeadDecay, channels = MODE == kChannelDelta;
+};
+
+// Forward walk of one row, head and block of value columns. OP: writes o and the final state; otherwise the checkpoints
+// and the residuals v_t - r_t that the gradients start from.
+template <typename T, int KL, int MODE, bool OP>
+__device__ __forceinline__ void forward_walk(const RecParams& p, WalkSmem<KL>& s, int r, int h, int v0) {
+  using W = Walk<MODE>;
+  const int K = p.K, V = p.V, hk = h / (p.H / p.Hk);
+  int tok0, len;
+  p.rows.range(r, tok0, len);
+  const Lane<KL> me(v0, V);
+  Chan S;
+  me.load_state(p.h0 ? p.h0 + ((long)r * p.H + h) * K * V : nullptr, K, V, S);
+  float* ckpt = nullptr;
+  if (!OP) {
+    const long slot = p.slot0(r, tok0);
+    ckpt = p.s_ckpt + ((long)h * p.slots + slot) * K * V;
+    if (h == 0 && v0 == 0) {
+      for (int b = threadIdx.x; b * TB < len; b += NW * 32) p.slot_row[slot + b] = r;
+    }
+  }
+  const float(*read_key)[WalkSmem<KL>::KP] = p.k_read ? s.kr : s.k;
+  Stage<T, KL> st;
+  st.load(p, static_cast<const T*>(p.v), OP, tok0, min(SB, len), tok0, h, hk, v0);
+  for (int t0 = 0; t0 < len; t0 += SB) {
+    const int nb = min(SB, len - t0);
+    __syncthreads();
+    st.commit(p, s, OP, nb);
+    __syncthreads();
+    if (t0 + SB < len) {
+      st.load(p, static_cast<const T*>(p.v), OP, tok0 + t0 + SB, min(SB, len - t0 - SB), tok0, h, hk, v0);
+    }
+    if (!OP && t0 % TB == 0) me.store_state(ckpt + (long)(t0 / TB) * K * V, K, V, S);
+    float out[SB];  // this thread's share of q_t S_t, or v_t - r_t
+    Chan e, w, k, q, e1, w1, k1, q1;  // this token's vectors and the next one's, read a token ahead of their use
+    auto fetch = [&](int j, Chan& e, Chan& w, Chan& k, Chan& q) {
+      if (W::channels) me.read(s.e[j], e);
+      if (W::delta) me.read(read_key[j], w);
+      me.read(s.k[j], k);
+      if (OP) me.read(s.q[j], q);
+    };
+    auto token = [&](int j, bool resets, Chan& e, Chan& w, Chan& k, Chan& q) {
+      if (resets && s.rs[j]) clear(S);
+      if (W::channels) scale_by(S, e);
+      else scale_by(S, s.es[j]);
+      float u = s.x[j][me.col];
+      if (W::delta) {
+        u -= key_sum<KL>(dot(w, S));
+        if (!OP) out[j] = u;
+        u *= s.bs[j];
+      }
+      axpy(S, k, u);
+      if (OP) out[j] = dot(q, S);
+    };
+    auto tokens = [&](auto with_resets) {
+      fetch(0, e, w, k, q);
+#pragma unroll
+      for (int j = 0; j < SB; j += 2) {
+        fetch(j + 1, e1, w1, k1, q1);
+        token(j, decltype(with_resets)::value, e, w, k, q);
+        if (j + 2 < SB) fetch(j + 2, e, w, k, q);
+        token(j + 1, decltype(with_resets)::value, e1, w1, k1, q1);
+      }
+    };
+    if (s.any_reset) tokens(std::true_type{});
+    else tokens(std::false_type{});
+    const long at = ((long)(tok0 + t0) * p.H + h) * V + me.v, next = (long)p.H * V;
+    if (OP) {
+#pragma unroll
+      for (int j = 0; j < SB; ++j) out[j] = key_sum<KL>(out[j]);
+    }
+    if ((OP || W::delta) && me.kl == 0 && me.active) {
+#pragma unroll
+      for (int j = 0; j < SB; ++j) {
+        if (j < nb) {
+          if (OP) static_cast<T*>(p.o)[at + j * next] = from_f32<T>(p.scale * out[j]);
+          else p.resid[at + j * next] = out[j];
+        }
+      }
+    }
+  }
+  if (OP) {
+    if (p.final_state) me.store_state(p.final_state + ((long)r * p.H + h) * K * V, K, V, S);
+  } else if (len > 0) {
+    me.store_state(ckpt + (long)((len + TB - 1) / TB) * K * V, K, V, S);
+  }
+}
+
+// Reverse walk of the state gradient, with a checkpoint of what comes from behind every block:
+//   dS += scale q_t^T do_t;  du_t = k_t dS;  dv_t = beta_t du_t, dr_t = -beta_t du_t;
+//   dS_{t-1} = exp(g_t) (dS + k_t^T dr_t)  (zero across a reset).
+template <typename T, int KL, int MODE>
+__device__ __forceinline__ void reverse_walk(const RecParams& p, WalkSmem<KL>& s, int r, int h, int v0) {
+  using W = Walk<MODE>;
+  const int K = p.K, V = p.V, hk = h / (p.H / p.Hk);
+  int tok0, len;
+  p.rows.range(r, tok0, len);
+  const Lane<KL> me(v0, V);
+  Chan dS;
+  me.load_state(p.d_final ? p.d_final + ((long)r * p.H + h) * K * V : nullptr, K, V, dS);
+  float* ckpt = p.ds_ckpt + ((long)h * p.slots + p.slot0(r, tok0)) * K * V;
+  const float(*read_key)[WalkSmem<KL>::KP] = p.k_read ? s.kr : s.k;
+  Stage<T, KL> st;
+  const int last = len > 0 ? (len - 1) / SB * SB : -SB;
+  if (len > 0) st.load(p, static_cast<const T*>(p.d_o), true, tok0 + last, len - last, tok0, h, hk, v0);
+  for (int t0 = last; t0 >= 0; t0 -= SB) {
+    const int nb = min(SB, len - t0);
+    __syncthreads();
+    st.commit(p, s, true, nb);
+    __syncthreads();
+    if (t0 > 0) st.load(p, static_cast<const T*>(p.d_o), true, tok0 + t0 - SB, SB, tok0, h, hk, v0);
+    if ((t0 + SB) % TB == 0 || t0 == last) me.store_state(ckpt + (long)(t0 / TB) * K * V, K, V, dS);
+    float out[SB];  // du_t
+    Chan e, w, k, q, e1, w1, k1, q1;
+    auto fetch = [&](int j, Chan& e, Chan& w, Chan& k, Chan& q) {
+      me.read(s.q[j], q);
+      me.read(s.k[j], k);
+      if (W::delta) me.read(read_key[j], w);
+      if (W::channels) me.read(s.e[j], e);
+    };
+    auto token = [&](int j, bool resets, Chan& e, Chan& w, Chan& k, Chan& q) {
+      axpy(dS, q, p.scale * s.x[j][me.col]);
+      out[j] = key_sum<KL>(dot(k, dS));
+      if (W::delta) axpy(dS, w, -s.bs[j] * out[j]);
+      if (W::channels) scale_by(dS, e);
+      else scale_by(dS, s.es[j]);
+      if (resets && s.rs[j]) clear(dS);
+    };
+    auto tokens = [&](auto with_resets) {
+      fetch(SB - 1, e, w, k, q);
+#pragma unroll
+      for (int j = SB - 1; j >= 0; j -= 2) {
+        fetch(j - 1, e1, w1, k1, q1);
+        token(j, decltype(with_resets)::value, e, w, k, q);
+        if (j >= 2) fetch(j - 2, e, w, k, q);
+        token(j - 1, decltype(with_resets)::value, e1, w1, k1, q1);
+      }
+    };
+    if (s.any_reset) tokens(std::true_type{});
+    else tokens(std::false_type{});
+    if (me.kl == 0 && me.active) {
+      const long at = ((long)(tok0 + t0) * p.H + h) * V + me.v, next = (long)p.H * V;
+#pragma unroll
+      for (int j = 0; j < SB; ++j) {
+        if (j < nb) {
+          static_cast<T*>(p.dv)[at + j * next] = from_f32<T>(W::delta ? s.bs[j] * out[j] : out[j]);
+          if (W::delta) p.du[at + j * next] = out[j];
+        }
+      }
+    }
+  }
+  if (p.dh0) me.store_state(p.dh0 + ((long)r * p.H + h) * K * V, K, V, dS);
+}
+
+// grid: (H * column blocks, rows)
+template <typename T, int KL, int MODE>
+__global__ void __launch_bounds__(NW * 32) rec_fwd_kernel(RecParams p) {
+  __shared__ __align__(16) WalkSmem<KL> s;
+  const int h = blockIdx.x % p.H, v0 = blockIdx.x / p.H * WalkSmem<KL>::NC;
+  forward_walk<T, KL, MODE, true>(p, s, blockIdx.y, h, v0);
+}
+
+// grid: (2 * H * column blocks, rows); the two walks are independent of each other
+template <typename T, int KL, int MODE>
+__global__ void __launch_bounds__(NW * 32) rec_bwd_kernel(RecParams p) {
+  __shared__ __align__(16) WalkSmem<KL> s;
+  const int x = blockIdx.x >> 1, h = x % p.H, v0 = x / p.H * WalkSmem<KL>::NC;
+  if (blockIdx.x & 1) reverse_walk<T, KL, MODE>(p, s, blockIdx.y, h, v0);
+  else forward_walk<T, KL, MODE, false>(p, s, blockIdx.y, h, v0);
+}
+
+// Gradients of q, k (and the read key) and of the gates for the TB tokens of one block and one head, from the state S0
+// entering the block, the state gradient dE coming from behind it and the per-token vectors do, dr = -beta du and
+// u = beta (v - r). With e_t the decay of token t (the products below stop at a reset):
+//   dq_t  = scale [ (prod_{s<=t} e_s) S0 do_t + sum_{j<=t} (prod_{j<s<=t} e_s) k_j (u_j . do_t) ]      (= scale S_t do_t)
+//   dkr_t =         (prod_{s<=t} e_s) S0 dr_t + sum_{j<t}  (prod_{j<s<=t} e_s) k_j (u_j . dr_t)        (= S'_t dr_t)
+//   dku_t = (prod_{s>t} e_s) dE u_t + sum_{i>=t} (prod_{t<s<=i} e_s) [scale q_i (do_i . u_t) + (i > t) kr_i (dr_i . u_t)]
+//   dbeta_t = du_t . (v_t - r_t);  dg_t = <dS'_t, S'_t> = (dg_{t+1}, or <dE, S_end> behind the block; zero across a reset)
+//             + q_t dq_t - k_t dku_t + kr_t dkr_t   per channel, summed over channels for scalar gates
+// Products of decays, never quotients, so any decay is safe. Latency hides behind the other blocks of the grid:
+// (tokens / TB) * H CTAs where the walks have one CTA per columns block.
+struct GradSmem {
+  int K, V, vs;  // K padded to whole channel tiles; vs: row stride of the value vectors
+  float *q, *k, *kr, *e, *d, *r, *u, *ts, *te, *tn, *ud, *ur, *udt, *urt, *es;
+  double *dl, *part;
+  __host__ __device__ static size_t floats(int K, int V) {
+    const int kp = (K + CT - 1) / CT * CT;
+    return 4 * TB * (size_t)kp + 3 * TB * (size_t)(V + 4) + 3 * CT * VTS + 4 * TB * TB + TB +
+           2 * (TB * CT + 4 * CT);
+  }
+  __device__ GradSmem(float* base, int k_dim, int v_dim) {
+    const int kp = (k_dim + CT - 1) / CT * CT;
+    K = kp, V = v_dim, vs = v_dim + 4;
+    q = base, k = q + TB * kp, kr = k + TB * kp, e = kr + TB * kp;
+    d = e + TB * kp, r = d + TB * vs, u = r + TB * vs;
+    ts = u + TB * vs, te = ts + CT * VTS, tn = te + CT * VTS;
+    ud = tn + CT * VTS, ur = ud + TB * TB, udt = ur + TB * TB, urt = udt + TB * TB, es = urt + TB * TB;
+    dl = reinterpret_cast<double*>(es + TB), part = dl + TB * CT;
+  }
+};
+
 template <typename T>
-__device__ void load_block(const RecParams& p, const Smem& s, int tok, int nb, int row_tok0, int h, int hk,
-                           bool with_do) {
-  const int K = p.K, V = p.V, NT = blockDim.x, tid = threadIdx.x;
-  const T* q = static_cast<const T*>(p.q);
-  const T* k = static_cast<const T*>(p.k);
-  const T* v = static_cast<const T*>(p.v);
-  for (int idx = tid; idx < nb * K; idx += NT) {
-    const int j = idx / K, c = idx - j * K;
-    const long src = ((long)(tok + j) * p.Hk + hk) * K + c;
-    s.qs[idx] = to_f32(q[src]);
-    s.ks[idx] = to_f32(k[src]);
-    if (p.k_read) s.kr[idx] = to_f32(static_cast<const T*>(p.k_read)[((long)(tok + j) * p.H + h) * K + c]);
-    if (p.gate == 2) s.eg[idx] = expf(p.g[((long)(tok + j) * p.H + h) * K + c]);
+__global__ void __launch_bounds__(GT) block_grads_kernel(RecParams p) {
+  extern __shared__ __align__(16) float smem_raw[];
+  const int K = p.K, V = p.V, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int h = blockIdx.x % p.H, hk = h / (p.H / p.Hk);
+  const long slot = blockIdx.x / p.H;
+  const int row = p.slot_row[slot];
+  if (row < 0 || row >= p.rows.count()) return;
+  int tok0, len;
+  p.rows.range(row, tok0, len);
+  const long b = slot - p.slot0(row, tok0);
+  if (b < 0 || b * TB >= len) return;
+  const int n = min(TB, len - (int)b * TB), tok = tok0 + (int)b * TB;
+  const GradSmem s(smem_raw, K, V);
+  __shared__ unsigned resets_s;
+
+  // ---- the block's vectors; tokens behind the row's end are zeros with decay 1
+#pragma unroll 4
+  for (int idx = tid; idx < TB * s.K; idx += GT) {
+    const int t = idx / s.K, c = idx - t * s.K;
+    const bool ok = t < n && c < K;
+    const long key = ((long)(tok + t) * p.Hk + hk) * K + c, kv = ((long)(tok + t) * p.H + h) * K + c;
+    const float k = ok ? to_f32(static_cast<const T*>(p.k)[key]) : 0.f;
+    s.q[idx] = ok ? to_f32(static_cast<const T*>(p.q)[key]) : 0.f;
+    s.k[idx] = k;
+    s.e[idx] = ok && p.gate == 2 ? expf(p.g[kv]) : 1.f;
+    s.kr[idx] = ok && p.k_read ? to_f32(static_cast<const T*>(p.k_read)[kv]) : k;
   }
-  for (int idx = tid; idx < nb * V; idx += NT) {
-    const int j = idx / V, c = idx - j * V;
-    const long src = ((long)(tok + j) * p.H + h) * V + c;
-    s.vs[idx] = to_f32(v[src]);
-    if (with_do) s.dos[idx] = to_f32(static_cast<const T*>(p.d_o)[src]);
+#pragma unroll 4
+  for (int idx = tid; idx < TB * V; idx += GT) {
+    const int t = idx / V, c = idx - t * V, at = t * s.vs + c;
+    const long src = ((long)(tok + t) * p.H + h) * V + c;
+    s.d[at] = t < n ? to_f32(static_cast<const T*>(p.d_o)[src]) : 0.f;
+    s.r[at] = t < n && p.delta ? p.du[src] : 0.f;
+    s.u[at] = t >= n ? 0.f : p.delta ? p.resid[src] : to_f32(static_cast<const T*>(p.v)[src]);
   }
-  if (tid < nb) {
-    const long src = (long)(tok + tid) * p.H + h;
-    if (p.gate == 1) s.eg[tid] = expf(p.g[src]);
-    s.bs[tid] = p.delta ? p.beta[src] : 1.f;
-    s.rs[tid] = p.rows.resets(tok + tid, row_tok0) ? 1 : 0;
+  if (warp == 0) {
+    const bool in = lane < n;
+    if (lane < TB) s.es[lane] = in && p.gate == 1 ? expf(p.g[(long)(tok + lane) * p.H + h]) : 1.f;
+    const unsigned bits = __ballot_sync(0xffffffffu, in && p.rows.resets(tok + lane, tok0));
+    if (lane == 0) resets_s = bits;
   }
   __syncthreads();
-  if (p.l2norm) {
-    if (tid < 2 * nb) {
-      const int which = tid / nb, j = tid - which * nb;
-      const float* x = (which ? s.ks : s.qs) + j * K;
-      float acc = 0.f;
-      for (int c = 0; c < K; ++c) acc += x[c] * x[c];
-      s.inv[which * TB + j] = rsqrtf(acc + 1e-6f);
-    }
-    __syncthreads();
-    for (int idx = tid; idx < nb * K; idx += NT) {
-      const int j = idx / K;
-      // the reference rounds the normalised tensors to the input dtype (reference.py:69)
-      s.qs[idx] = to_f32(from_f32<T>(s.qs[idx] * s.inv[j]));
-      s.ks[idx] = to_f32(from_f32<T>(s.ks[idx] * s.inv[TB + j]));
+  if (p.l2norm || p.delta) {
+    for (int t = warp; t < n; t += GT / 32) {
+      if (p.l2norm) {  // the reference rounds the normalised tensors to the input dtype (reference.py:69)
+        float sq = 0.f, sk = 0.f;
+        for (int c = lane; c < s.K; c += 32) {
+          const float q = s.q[t * s.K + c], k = s.k[t * s.K + c];
+          sq += q * q, sk += k * k;
+        }
+        const float iq = rsqrtf(warp_sum(sq) + 1e-6f), ik = rsqrtf(warp_sum(sk) + 1e-6f);
+        for (int c = lane; c < s.K; c += 32) {
+          s.q[t * s.K + c] = to_f32(from_f32<T>(s.q[t * s.K + c] * iq));
+          s.k[t * s.K + c] = to_f32(from_f32<T>(s.k[t * s.K + c] * ik));
+          if (!p.k_read) s.kr[t * s.K + c] = s.k[t * s.K + c];
+        }
+      }
+      if (p.delta) {  // du, v - r  ->  -beta du, beta (v - r), and their product's sum on the way
+        const long th = (long)(tok + t) * p.H + h;
+        const float beta = p.beta[th];
+        float db = 0.f;
+        for (int c = lane; c < V; c += 32) {
+          const float du = s.r[t * s.vs + c], x = s.u[t * s.vs + c];
+          s.r[t * s.vs + c] = -beta * du, s.u[t * s.vs + c] = beta * x;
+          db += du * x;
+        }
+        db = warp_sum(db);
+        if (lane == 0) p.dbeta[th] = db;
+      }
     }
     __syncthreads();
   }
-  if (!p.k_read) {  // the write key is also the read key (after its normalisation)
-    for (int idx = tid; idx < nb * K; idx += NT) s.kr[idx] = s.ks[idx];
-    __syncthreads();
-  }
-}
+  const unsigned resets = resets_s;
 
-// One forward token: reset, decay, (delta) recall and write. Returns the written value u_v; *resid gets
-// v_v - r_v. Contains one __syncthreads() when delta is set.
-template <int KPT>
-__device__ __forceinline__ float forward_token(const RecParams& p, const Smem& s, float (&S)[KPT], int j, int ks,
-                                               int v, int KS, float* resid, float* pre /*global or nullptr*/) {
-  const int K = p.K, V = p.V;
-  if (s.rs[j]) {
+  {  // u_j . do_t and u_j . dr_t, one pair (j, t) a thread
+    const int j = tid / TB, t = tid % TB;
+    float at = 0.f, ct = 0.f;
+    for (int x0 = 0; x0 < V; x0 += VT) {  // (sums of short sums: the rounding of a long chain would show in dg)
+      float a[4] = {}, c[4] = {};
+#pragma unroll 4
+      for (int x = x0; x < min(V, x0 + VT); x += 4) {
+        const float4 u = *reinterpret_cast<const float4*>(s.u + j * s.vs + x);
+        const float4 d = *reinterpret_cast<const float4*>(s.d + t * s.vs + x);
+        const float4 r = *reinterpret_cast<const float4*>(s.r + t * s.vs + x);
+        a[0] += u.x * d.x, a[1] += u.y * d.y, a[2] += u.z * d.z, a[3] += u.w * d.w;
+        c[0] += u.x * r.x, c[1] += u.y * r.y, c[2] += u.z * r.z, c[3] += u.w * r.w;
+      }
+      at += (a[0] + a[1]) + (a[2] + a[3]), ct += (c[0] + c[1]) + (c[2] + c[3]);
+    }
+    s.udt[t * TB + j] = s.ud[tid] = at;
+    s.urt[t * TB + j] = s.ur[tid] = ct;
+  }
+
+  const float* S0 = p.s_ckpt + ((long)h * p.slots + slot) * K * V;
+  const float* dE = p.ds_ckpt + ((long)h * p.slots + slot) * K * V;
+  const int cl = tid % CT, tg = tid / CT, tq = 4 * tg;  // channel of the tile; this thread's tokens are tq .. tq + 3
+  double gsum[4] = {}, gend = 0.;                       // scalar gates: this thread's channels' share of the dg terms
+  for (int c0 = 0; c0 < K; c0 += CT) {
+    // ---- S0 do_t, S0 dr_t, dE u_t for the tile's channels, and <dE, S_end>
+    float ad[4] = {}, ar[4] = {}, au[4] = {}, en = 0.f;
+    for (int x0 = 0; x0 < V; x0 += VT) {
+      __syncthreads();
 #pragma unroll
-    for (int i = 0; i < KPT; ++i) S[i] = 0.f;
+      for (int idx = tid; idx < CT * VT / 4; idx += GT) {
+        const int c = idx / (VT / 4), x = idx % (VT / 4) * 4;
+        const bool ok = c0 + c < K && x0 + x < V;
+        const long at = (long)(c0 + c) * V + x0 + x;
+        const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+        *reinterpret_cast<float4*>(s.ts + c * VTS + x) = ok ? *reinterpret_cast<const float4*>(S0 + at) : z;
+        *reinterpret_cast<float4*>(s.te + c * VTS + x) = ok ? *reinterpret_cast<const float4*>(dE + at) : z;
+        *reinterpret_cast<float4*>(s.tn + c * VTS + x) =
+            ok && p.gate ? *reinterpret_cast<const float4*>(S0 + (long)K * V + at) : z;
+      }
+      __syncthreads();
+      const int xe = min(VT, V - x0);
+      float td[4] = {}, tr[4] = {}, tu[4] = {}, tn = 0.f;
+      for (int x = 0; x < xe; x += 4) {
+        const float4 a = *reinterpret_cast<const float4*>(s.ts + cl * VTS + x);
+        const float4 g = *reinterpret_cast<const float4*>(s.te + cl * VTS + x);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int at = (tq + i) * s.vs + x0 + x;
+          const float4 d = *reinterpret_cast<const float4*>(s.d + at);
+          const float4 r = *reinterpret_cast<const float4*>(s.r + at);
+          const float4 u = *reinterpret_cast<const float4*>(s.u + at);
+          td[i] += (a.x * d.x + a.y * d.y) + (a.z * d.z + a.w * d.w);
+          tr[i] += (a.x * r.x + a.y * r.y) + (a.z * r.z + a.w * r.w);
+          tu[i] += (g.x * u.x + g.y * u.y) + (g.z * u.z + g.w * u.w);
+        }
+        if ((x / 4 & 3) == tg) {
+          const float4 e = *reinterpret_cast<const float4*>(s.tn + cl * VTS + x);
+          tn += (g.x * e.x + g.y * e.y) + (g.z * e.z + g.w * e.w);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) ad[i] += td[i], ar[i] += tr[i], au[i] += tu[i];
+      en += tn;
+    }
+    // ---- the in-block terms of this thread's channel and four tokens; the products of decays grow one token at a time.
+    // The term that token t's own write and read share (q_t . k_t)(u_t . do_t) cancels in dg and joins after it.
+    const int c = c0 + cl;
+    float w[4] = {1.f, 1.f, 1.f, 1.f}, dq[4] = {}, dkr[4] = {}, dk[4] = {};
+#pragma unroll 4
+    for (int j = TB - 1; j >= 0; --j) {  // from token j's predecessor (or the entering state) into tokens t >= j
+      const float e = p.gate == 2 ? s.e[j * s.K + c] : s.es[j];
+      const bool cut = resets >> j & 1;
+      const float kp = j > 0 ? s.k[(j - 1) * s.K + c] : 0.f;
+      const int at = (j > 0 ? j - 1 : 0) * TB + tq;
+      const float4 x = *reinterpret_cast<const float4*>(s.ud + at), y = *reinterpret_cast<const float4*>(s.ur + at);
+      const float xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (tq + i >= j) {
+          w[i] = cut ? 0.f : w[i] * e;
+          if (w[i] != 0.f) dq[i] += w[i] * kp * xs[i], dkr[i] += w[i] * kp * ys[i];
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (w[i] != 0.f) dq[i] += w[i] * ad[i], dkr[i] += w[i] * ar[i];
+      w[i] = 1.f;
+    }
+#pragma unroll 4
+    for (int j = 1; j < TB; ++j) {  // what tokens j > t read of token t's write
+      const float e = p.gate == 2 ? s.e[j * s.K + c] : s.es[j];
+      const bool cut = resets >> j & 1;
+      const float qj = p.scale * s.q[j * s.K + c], rj = s.kr[j * s.K + c];
+      const float4 x = *reinterpret_cast<const float4*>(s.udt + j * TB + tq);
+      const float4 y = *reinterpret_cast<const float4*>(s.urt + j * TB + tq);
+      const float xs[4] = {x.x, x.y, x.z, x.w}, ys[4] = {y.x, y.y, y.z, y.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        if (tq + i < j) {
+          w[i] = cut ? 0.f : w[i] * e;
+          if (w[i] != 0.f) dk[i] += w[i] * (qj * xs[i] + rj * ys[i]);
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int t = tq + i;
+      const float q = s.q[t * s.K + c], k = s.k[t * s.K + c], own = s.ud[t * TB + t];
+      if (w[i] != 0.f) dk[i] += w[i] * au[i];
+      // (the terms of dg are much larger than their sum: they are added up in 64 bits)
+      const double x = (double)(p.scale * q) * dq[i] - (double)k * dk[i] + (double)s.kr[t * s.K + c] * dkr[i];
+      if (p.gate == 2) s.dl[t * CT + cl] = x;
+      else gsum[i] += x;
+      if (t < n && c < K) {
+        const long at = ((long)(tok + t) * p.H + h) * K + c;
+        const float dku = dk[i] + p.scale * q * own;
+        p.dq_acc[at] = p.scale * (dq[i] + k * own);
+        p.dk_acc[at] = p.k_read ? dku : dku + dkr[i];
+        if (p.k_read) p.dkr_acc[at] = dkr[i];
+      }
+    }
+    if (p.gate == 2) {
+      s.part[tg * CT + cl] = en;
+      __syncthreads();
+      if (tid < CT && c < K) {
+        double carry = (s.part[cl] + s.part[CT + cl]) + (s.part[2 * CT + cl] + s.part[3 * CT + cl]);
+        for (int t = n - 1; t >= 0; --t) {
+          carry += s.dl[t * CT + cl];
+          if (resets >> t & 1) carry = 0.;
+          p.dg[((long)(tok + t) * p.H + h) * K + c] = (float)carry;
+        }
+      }
+    } else {
+      gend += en;
+    }
   }
   if (p.gate == 1) {
-    const float d = s.eg[j];
 #pragma unroll
-    for (int i = 0; i < KPT; ++i) S[i] *= d;
-  } else if (p.gate == 2) {
+    for (int i = 0; i < 4; ++i) gsum[i] = warp_sum(gsum[i]);
+    gend = warp_sum(gend);
+    if (lane == 0) {  // warps 2 tg and 2 tg + 1 hold the two halves of a channel tile for tokens tq .. tq + 3
 #pragma unroll
-    for (int i = 0; i < KPT; ++i) S[i] *= s.eg[j * K + ks * KPT + i];
-  }
-  if (pre) {
-#pragma unroll
-    for (int i = 0; i < KPT; ++i) pre[(long)(ks * KPT + i) * V + v] = S[i];
-  }
-  float u = s.vs[j * V + v];
-  if (p.delta) {
-    float partial = 0.f;
-#pragma unroll
-    for (int i = 0; i < KPT; ++i) partial += s.kr[j * K + ks * KPT + i] * S[i];
-    float* part_r = s.part + 2 * KS * V;
-    part_r[ks * V + v] = partial;
+      for (int i = 0; i < 4; ++i) s.dl[(warp & 1) * TB + tq + i] = gsum[i];
+      s.part[warp] = gend;
+    }
     __syncthreads();
-    float r = 0.f;
-    for (int t = 0; t < KS; ++t) r += part_r[t * V + v];
-    *resid = u - r;
-    u = s.bs[j] * (u - r);
-  }
-#pragma unroll
-  for (int i = 0; i < KPT; ++i) S[i] += s.ks[j * K + ks * KPT + i] * u;
-  return u;
-}
-
-template <typename T, int KPT>
-__global__ void __launch_bounds__(512) rec_fwd_kernel(RecParams p) {
-  extern __shared__ float smem_raw[];
-  const int h = blockIdx.x, r = blockIdx.y;
-  const int K = p.K, V = p.V, tid = threadIdx.x;
-  const int v = tid % V, ks = tid / V, KS = K / KPT;
-  const int hk = h / (p.H / p.Hk);
-  const Smem s = carve(smem_raw, K, V, KS, false);
-  int tok0, len;
-  p.rows.range(r, tok0, len);
-
-  float S[KPT];
-  const float* h0 = p.h0 ? p.h0 + ((long)r * p.H + h) * K * V : nullptr;
-#pragma unroll
-  for (int i = 0; i < KPT; ++i) S[i] = h0 ? h0[(long)(ks * KPT + i) * V + v] : 0.f;
-
-  T* o = static_cast<T*>(p.o);
-  for (int t0 = 0; t0 < len; t0 += TB) {
-    const int nb = min(TB, len - t0);
-    __syncthreads();
-    load_block<T>(p, s, tok0 + t0, nb, tok0, h, hk, false);
-    for (int j = 0; j < nb; ++j) {
-      float resid;
-      forward_token<KPT>(p, s, S, j, ks, v, KS, &resid, nullptr);
-      float po = 0.f;
-#pragma unroll
-      for (int i = 0; i < KPT; ++i) po += s.qs[j * K + ks * KPT + i] * S[i];
-      float* part_o = s.part + (j & 1) * KS * V;
-      part_o[ks * V + v] = po;
-      __syncthreads();
-      if (ks == 0) {
-        float acc = 0.f;
-        for (int t = 0; t < KS; ++t) acc += part_o[t * V + v];
-        o[((long)(tok0 + t0 + j) * p.H + h) * V + v] = from_f32<T>(p.scale * acc);
+    if (tid == 0) {
+      double carry = 0.;
+      for (int w = 0; w < GT / 32; ++w) carry += s.part[w];
+      for (int t = n - 1; t >= 0; --t) {
+        carry += s.dl[t] + s.dl[TB + t];
+        if (resets >> t & 1) carry = 0.;
+        p.dg[(long)(tok + t) * p.H + h] = (float)carry;
       }
     }
   }
-  if (p.final_state) {
-    float* f = p.final_state + ((long)r * p.H + h) * K * V;
-#pragma unroll
-    for (int i = 0; i < KPT; ++i) f[(long)(ks * KPT + i) * V + v] = S[i];
-  }
 }
 
-// Sum val[i] over the value columns of this key slice; lane v % 32 == 0 of every warp writes its partial to
-// red[(v / 32) * K + key]. V is a power of two, so a shuffle tree of width min(V, 32) stays inside the slice.
-template <int KPT>
-__device__ __forceinline__ void reduce_over_v(const float (&val)[KPT], float* red, int K, int V, int ks, int v) {
-  const int width = V < 32 ? V : 32;
-#pragma unroll
-  for (int i = 0; i < KPT; ++i) {
-    float x = val[i];
-    for (int off = width >> 1; off > 0; off >>= 1) x += __shfl_xor_sync(0xffffffffu, x, off);
-    if ((v & (width - 1)) == 0) red[(v >> 5) * K + ks * KPT + i] = x;
+// Head sizes of the path: V columns times slices of 1, 2, 4 .. 128 key channels in at most 512 threads, whole warps.
+bool covered(int K, int V) {
+  for (int slice = 1; slice <= 128; slice *= 2) {
+    if (K % slice == 0 && (long)V * (K / slice) <= 512 && V * (K / slice) % 32 == 0) return true;
   }
+  return false;
 }
 
-// Backward of the token scan. Phase A re-runs the forward and checkpoints the state entering every TB-token
-// block; phase B walks the blocks in reverse, re-materialises the post-decay states S'_t of one block into
-// `spre` (each thread writes and later reads only its own entries) and then walks its tokens backwards:
-//   dS += scale q_t^T do_t;  dq_t = scale S_t do_t;  du_t = k_t dS;  dk_t = dS u_t (+ S'_t dr_t);
-//   delta: dbeta_t = du_t . (v_t - r_t), dv_t = beta_t du_t, dr_t = -beta_t du_t, dS' = dS + k_t^T dr_t;
-//   dg_t = <dS', S'_t> (per channel for vector gates);  dS_{t-1} = exp(g_t) dS' (zero across a reset).
-template <typename T, int KPT>
-__global__ void __launch_bounds__(512) rec_bwd_kernel(RecParams p) {
-  extern __shared__ float smem_raw[];
-  const int h = blockIdx.x, r = blockIdx.y;
-  const int K = p.K, V = p.V, tid = threadIdx.x;
-  const int v = tid % V, ks = tid / V, KS = K / KPT;
-  const int hk = h / (p.H / p.Hk);
-  const int VW = V < 32 ? 1 : V / 32;
-  const Smem s = carve(smem_raw, K, V, KS, true);
-  int tok0, len;
-  p.rows.range(r, tok0, len);
-  const int nblk = (len + TB - 1) / TB;
-  float* ckpt = p.ckpt + ((long)h * p.total_blocks + tok0 / TB + r) * K * V;
-  float* spre = p.spre + ((long)r * p.H + h) * TB * K * V;
-
-  float S[KPT];
-  const float* h0 = p.h0 ? p.h0 + ((long)r * p.H + h) * K * V : nullptr;
-#pragma unroll
-  for (int i = 0; i < KPT; ++i) S[i] = h0 ? h0[(long)(ks * KPT + i) * V + v] : 0.f;
-
-  // ---- phase A: checkpoints
-  for (int b = 0; b < nblk; ++b) {
-    const int t0 = b * TB, nb = min(TB, len - t0);
-#pragma unroll
-    for (int i = 0; i < KPT; ++i) ckpt[(long)b * K * V + (long)(ks * KPT + i) * V + v] = S[i];
-    if (b == nblk - 1) break;
-    __syncthreads();
-    load_block<T>(p, s, tok0 + t0, nb, tok0, h, hk, false);
-    for (int j = 0; j < nb; ++j) {
-      float resid;
-      forward_token<KPT>(p, s, S, j, ks, v, KS, &resid, nullptr);
-      if (!p.delta) continue;
-      __syncthreads();  // part_r is rewritten by the next token
-    }
-  }
-
-  // ---- phase B
-  float dS[KPT];
-  const float* dfin = p.d_final ? p.d_final + ((long)r * p.H + h) * K * V : nullptr;
-#pragma unroll
-  for (int i = 0; i < KPT; ++i) dS[i] = dfin ? dfin[(long)(ks * KPT + i) * V + v] : 0.f;
-
-  T* dv = static_cast<T*>(p.dv);
-  for (int b = nblk - 1; b >= 0; --b) {
-    const int t0 = b * TB, nb = min(TB, len - t0);
-#pragma unroll
-    for (int i = 0; i < KPT; ++i) S[i] = ckpt[(long)b * K * V + (long)(ks * KPT + i) * V + v];
-    __syncthreads();
-    load_block<T>(p, s, tok0 + t0, nb, tok0, h, hk, true);
-    for (int j = 0; j < nb; ++j) {
-      float resid = 0.f;
-      const float u = forward_token<KPT>(p, s, S, j, ks, v, KS, &resid, spre + (long)j * K * V);
-      if (ks == 0) {
-        s.us[j * V + v] = u;
-        s.es[j * V + v] = resid;
-      }
-      if (p.delta) __syncthreads();
-    }
-    __syncthreads();
-
-    for (int j = nb - 1; j >= 0; --j) {
-      const long tok = tok0 + t0 + j;
-      float* red = s.red + (j & 1) * (4 * 8 * K + 64);
-      float* red_q = red;
-      float* red_k = red + 8 * K;
-      float* red_g = red + 16 * K;
-      float* red_s = red + 24 * K;  // [0..31] dbeta partials, [32..63] scalar dg partials (per warp, <= 16 warps)
-      float* red_kr = red + 24 * K + 64;
-      float Sp[KPT], tmp[KPT];
-      const float u = s.us[j * V + v];
-      const float dov = s.dos[j * V + v];
-#pragma unroll
-      for (int i = 0; i < KPT; ++i) {
-        const float ki = s.ks[j * K + ks * KPT + i];
-        Sp[i] = spre[(long)j * K * V + (long)(ks * KPT + i) * V + v];
-        tmp[i] = (Sp[i] + ki * u) * dov;                      // S_t[k, v] do_v
-        dS[i] += p.scale * s.qs[j * K + ks * KPT + i] * dov;  // o_t = scale q_t S_t
-      }
-      reduce_over_v<KPT>(tmp, red_q, K, V, ks, v);
-      float partial = 0.f;
-#pragma unroll
-      for (int i = 0; i < KPT; ++i) partial += s.ks[j * K + ks * KPT + i] * dS[i];
-      float* part_r = s.part + 2 * KS * V;
-      part_r[ks * V + v] = partial;
-      __syncthreads();  // #1
-      float du = 0.f;
-      for (int t = 0; t < KS; ++t) du += part_r[t * V + v];
-      const float beta = s.bs[j];
-      const float dr = p.delta ? -beta * du : 0.f;
-      float tmpr[KPT];  // the read key's gradient S'_t dr_t; added to dk when the write key is also the read key
-#pragma unroll
-      for (int i = 0; i < KPT; ++i) {
-        tmpr[i] = Sp[i] * dr;
-        tmp[i] = dS[i] * u + (p.k_read ? 0.f : tmpr[i]);
-      }
-      reduce_over_v<KPT>(tmp, red_k, K, V, ks, v);
-      if (p.k_read) reduce_over_v<KPT>(tmpr, red_kr, K, V, ks, v);
-      if (ks == 0) dv[(tok * p.H + h) * V + v] = from_f32<T>(p.delta ? beta * du : du);
-      if (p.delta) {  // dbeta_t = sum_v du_v (v_v - r_v): reduce over the ks == 0 threads (warps 0 .. VW-1)
-        float x = ks == 0 ? du * s.es[j * V + v] : 0.f;
-        for (int off = 16; off > 0; off >>= 1) x += __shfl_xor_sync(0xffffffffu, x, off);
-        if ((tid & 31) == 0 && tid < V) red_s[tid >> 5] = x;
-      }
-      float gsum = 0.f;
-#pragma unroll
-      for (int i = 0; i < KPT; ++i) {
-        const float dSp = dS[i] + s.kr[j * K + ks * KPT + i] * dr;  // gradient of S'_t
-        tmp[i] = dSp * Sp[i];
-        gsum += tmp[i];
-        const float decay = p.gate == 1 ? s.eg[j] : (p.gate == 2 ? s.eg[j * K + ks * KPT + i] : 1.f);
-        dS[i] = s.rs[j] ? 0.f : decay * dSp;
-      }
-      if (p.gate == 2) reduce_over_v<KPT>(tmp, red_g, K, V, ks, v);
-      if (p.gate == 1) {
-        for (int off = 16; off > 0; off >>= 1) gsum += __shfl_xor_sync(0xffffffffu, gsum, off);
-        if ((tid & 31) == 0) red_s[32 + (tid >> 5)] = gsum;
-      }
-      __syncthreads();  // #2
-      if (tid < K) {
-        float aq = 0.f, ak = 0.f, ag = 0.f, akr = 0.f;
-        for (int w = 0; w < VW; ++w) {
-          aq += red_q[w * K + tid];
-          ak += red_k[w * K + tid];
-          if (p.gate == 2) ag += red_g[w * K + tid];
-          if (p.k_read) akr += red_kr[w * K + tid];
-        }
-        p.dq_acc[(tok * p.H + h) * K + tid] = p.scale * aq;
-        p.dk_acc[(tok * p.H + h) * K + tid] = ak;
-        if (p.k_read) p.dkr_acc[(tok * p.H + h) * K + tid] = akr;
-        if (p.gate == 2) p.dg[(tok * p.H + h) * K + tid] = ag;
-      }
-      if (tid == 0) {
-        if (p.delta) {
-          float x = 0.f;
-          for (int w = 0; w < VW; ++w) x += red_s[w];
-          p.dbeta[tok * p.H + h] = x;
-        }
-        if (p.gate == 1) {
-          float x = 0.f;
-          for (int w = 0; w < (int)(blockDim.x >> 5); ++w) x += red_s[32 + w];
-          p.dg[tok * p.H + h] = x;
-        }
-      }
-    }
-  }
-  if (p.dh0) {
-    float* out = p.dh0 + ((long)r * p.H + h) * K * V;
-#pragma unroll
-    for (int i = 0; i < KPT; ++i) out[(long)(ks * KPT + i) * V + v] = dS[i];
-  }
-}
-
-int pick_kpt(int K, int V) {
-  for (int kpt = 1; kpt <= 128; kpt *= 2) {
-    if (K % kpt) continue;
-    const long nt = (long)V * (K / kpt);
-    if (nt <= 512 && nt % 32 == 0) return kpt;
-  }
-  return 0;
-}
+// Key lanes per column: 16 channels a thread.
+int pick_key_lanes(int K) { return K <= 32 ? 2 : K <= 64 ? 4 : K <= 128 ? 8 : 16; }
 
 RecParams base_params(const jla_problem& p) {
   RecParams r{};
@@ -401,50 +746,51 @@ RecParams base_params(const jla_problem& p) {
   return r;
 }
 
-template <typename T, int KPT>
-int launch(const RecParams& rp, bool bwd, int rows, cudaStream_t stream) {
-  const int KS = rp.K / KPT;
-  const size_t smem = smem_floats(rp.K, rp.V, KS, bwd) * sizeof(float);
-  auto* kern = bwd ? rec_bwd_kernel<T, KPT> : rec_fwd_kernel<T, KPT>;
-  if (smem > 48 * 1024) JLA_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  dim3 grid(rp.H, rows), block(rp.V * KS);
-  {
-    ProfScope ps(bwd ? kProfRecBwd : kProfRecFwd, stream);
-    kern<<<grid, block, smem, stream>>>(rp);
-  }
+template <typename T, int KL>
+int launch_walks(const RecParams& rp, bool bwd, int rows, cudaStream_t stream) {
+  const int blocks = (rp.V + WalkSmem<KL>::NC - 1) / WalkSmem<KL>::NC;
+  ProfScope ps(bwd ? kProfRecBwd : kProfRecFwd, stream);
+  const dim3 grid((unsigned)(rp.H * blocks * (bwd ? 2 : 1)), (unsigned)rows);
+  auto run = [&](auto* fwd, auto* back) { (bwd ? back : fwd)<<<grid, NW * 32, 0, stream>>>(rp); };
+  if (!rp.delta) run(rec_fwd_kernel<T, KL, kHeadDecay>, rec_bwd_kernel<T, KL, kHeadDecay>);
+  else if (rp.gate == 2) run(rec_fwd_kernel<T, KL, kChannelDelta>, rec_bwd_kernel<T, KL, kChannelDelta>);
+  else run(rec_fwd_kernel<T, KL, kHeadDelta>, rec_bwd_kernel<T, KL, kHeadDelta>);
   JLA_LAUNCH_OK();
   return JLA_OK;
 }
 
 template <typename T>
-int launch_kpt(const RecParams& rp, int kpt, bool bwd, int rows, cudaStream_t stream) {
-  switch (kpt) {
-    case 1: return launch<T, 1>(rp, bwd, rows, stream);
-    case 2: return launch<T, 2>(rp, bwd, rows, stream);
-    case 4: return launch<T, 4>(rp, bwd, rows, stream);
-    case 8: return launch<T, 8>(rp, bwd, rows, stream);
-    case 16: return launch<T, 16>(rp, bwd, rows, stream);
-    case 32: return launch<T, 32>(rp, bwd, rows, stream);
-    case 64: return launch<T, 64>(rp, bwd, rows, stream);
-    case 128: return launch<T, 128>(rp, bwd, rows, stream);
+int launch_t(const RecParams& rp, bool bwd, int rows, cudaStream_t stream) {
+  int rc;
+  switch (pick_key_lanes(rp.K)) {
+    case 2: rc = launch_walks<T, 2>(rp, bwd, rows, stream); break;
+    case 4: rc = launch_walks<T, 4>(rp, bwd, rows, stream); break;
+    case 8: rc = launch_walks<T, 8>(rp, bwd, rows, stream); break;
+    default: rc = launch_walks<T, 16>(rp, bwd, rows, stream); break;
   }
-  set_error("recurrent path: no thread layout for K=%d V=%d", rp.K, rp.V);
-  return JLA_ERR_UNSUPPORTED;
+  if (rc != JLA_OK || !bwd) return rc;
+  const size_t smem = GradSmem::floats(rp.K, rp.V) * sizeof(float);
+  JLA_CUDA_OK(cudaFuncSetAttribute(block_grads_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  ProfScope ps(kProfRecGrads, stream);
+  block_grads_kernel<T><<<(unsigned)(rp.slots * rp.H), GT, smem, stream>>>(rp);
+  JLA_LAUNCH_OK();
+  return JLA_OK;
 }
 
-int launch_dtype(const RecParams& rp, int dtype, int kpt, bool bwd, int rows, cudaStream_t stream) {
+int launch_dtype(const RecParams& rp, int dtype, bool bwd, int rows, cudaStream_t stream) {
   switch (dtype) {
-    case JLA_DTYPE_BF16: return launch_kpt<__nv_bfloat16>(rp, kpt, bwd, rows, stream);
-    case JLA_DTYPE_F16: return launch_kpt<__half>(rp, kpt, bwd, rows, stream);
-    case JLA_DTYPE_F32: return launch_kpt<float>(rp, kpt, bwd, rows, stream);
+    case JLA_DTYPE_BF16: return launch_t<__nv_bfloat16>(rp, bwd, rows, stream);
+    case JLA_DTYPE_F16: return launch_t<__half>(rp, bwd, rows, stream);
+    case JLA_DTYPE_F32: return launch_t<float>(rp, bwd, rows, stream);
   }
   set_error("unknown dtype %d", dtype);
   return JLA_ERR_BAD_ARGUMENT;
 }
 
 struct BwdScratch {
-  float *dq_acc, *dk_acc, *dkr_acc, *ckpt, *spre;
-  long total_blocks;
+  float *dq_acc, *dk_acc, *dkr_acc, *s_ckpt, *ds_ckpt, *resid, *du;
+  int* slot_row;
+  long slots;
   size_t bytes;
 };
 
@@ -453,12 +799,16 @@ BwdScratch carve_bwd(const jla_problem& p, void* base) {
   BwdScratch s;
   const long tokens = (long)p.B * p.T;
   const int rows = p.cu_seqlens || p.num_seqs ? p.num_seqs : p.B;
-  s.total_blocks = tokens / TB + rows + 1;
+  const bool delta = p.kind != JLA_KIND_SIMPLE_GLA;
+  s.slots = tokens / TB + 2L * rows + 1;
   s.dq_acc = c.take<float>((size_t)tokens * p.H * p.K);
   s.dk_acc = c.take<float>((size_t)tokens * p.H * p.K);
   s.dkr_acc = c.take<float>(p.k_read ? (size_t)tokens * p.H * p.K : 0);
-  s.ckpt = c.take<float>((size_t)p.H * s.total_blocks * p.K * p.V);
-  s.spre = c.take<float>((size_t)rows * p.H * TB * p.K * p.V);
+  s.s_ckpt = c.take<float>((size_t)p.H * s.slots * p.K * p.V);
+  s.ds_ckpt = c.take<float>((size_t)p.H * s.slots * p.K * p.V);
+  s.resid = c.take<float>(delta ? (size_t)tokens * p.H * p.V : 0);
+  s.du = c.take<float>(delta ? (size_t)tokens * p.H * p.V : 0);
+  s.slot_row = c.take<int>((size_t)s.slots);
   s.bytes = c.bytes();
   return s;
 }
@@ -468,7 +818,7 @@ BwdScratch carve_bwd(const jla_problem& p, void* base) {
 const char* recurrent_unsupported(const jla_problem& p) {
   if (p.K > 256 || p.V > 256 || p.K % 8) return "recurrent path: K must be a multiple of 8 and K, V <= 256";
   if (p.V < 8 || (p.V & (p.V - 1))) return "recurrent path: V must be a power of two in [8, 256]";
-  if (!pick_kpt(p.K, p.V)) return "recurrent path: no thread layout for this K, V";
+  if (!covered(p.K, p.V)) return "recurrent path: no thread layout for this K, V";
   return nullptr;
 }
 
@@ -480,7 +830,7 @@ int recurrent_fwd(const jla_problem& p, const jla_fwd_io& io, cudaStream_t strea
   rp.final_state = io.final_state;
   const int rows = p.cu_seqlens ? p.num_seqs : p.B;
   if (rows == 0 || p.H == 0) return JLA_OK;
-  return launch_dtype(rp, p.dtype, pick_kpt(p.K, p.V), false, rows, stream);
+  return launch_dtype(rp, p.dtype, false, rows, stream);
 }
 
 int recurrent_bwd(const jla_problem& p, const jla_bwd_io& io, cudaStream_t stream) {
@@ -493,11 +843,12 @@ int recurrent_bwd(const jla_problem& p, const jla_bwd_io& io, cudaStream_t strea
   rp.d_o = io.d_o; rp.d_final = io.d_final;
   rp.dq_acc = s.dq_acc; rp.dk_acc = s.dk_acc; rp.dkr_acc = s.dkr_acc;
   rp.dv = io.dv; rp.dg = io.dg; rp.dbeta = io.dbeta; rp.dh0 = io.dh0;
-  rp.ckpt = s.ckpt; rp.spre = s.spre; rp.total_blocks = s.total_blocks;
+  rp.s_ckpt = s.s_ckpt; rp.ds_ckpt = s.ds_ckpt; rp.resid = s.resid; rp.du = s.du;
+  rp.slot_row = s.slot_row; rp.slots = s.slots;
   const int rows = p.cu_seqlens ? p.num_seqs : p.B;
   const long tokens = (long)p.B * p.T;
   if (rows > 0 && p.H > 0) {
-    const int rc = launch_dtype(rp, p.dtype, pick_kpt(p.K, p.V), true, rows, stream);
+    const int rc = launch_dtype(rp, p.dtype, true, rows, stream);
     if (rc != JLA_OK) return rc;
   }
   const bool l2 = (p.flags & JLA_FLAG_QK_L2NORM) != 0;
