@@ -28,6 +28,7 @@ struct Plan {
   size_t meta, row_chunks, gates, runs, t0, ag, qn, kn, h, vn, w, residual_bytes;  // residual buffer
   size_t kda_q, kda_kr, kda_kw, kda_p, kda_d;  // KDA: gate-folded operands per chunk slot (see chunked_kda_prep.cu)
   size_t qk_tab;  // grouped simple GLA on the mma.sync kernels: Q K^T and K Q^T per (chunk, key head), see qk_table_kernel
+  size_t z;  // backward of the split kernels: scale P^T dO in fp32, see chunked_split.cu
   size_t kda_dag, kda_dqs, kda_dks, kda_dku, kda_dd;  // KDA backward scratch (see chunked_kda_bwd.cu)
   size_t fwd_scratch_bytes;                                                 // same layout without h, vn
   size_t dh, dvn, dq_acc, dk_acc, dp, dga, bwd_scratch_bytes;               // backward scratch
@@ -114,6 +115,7 @@ inline Plan make_plan(const jla_problem& p) {
   pl.dk_acc = boff(direct ? 0 : tokens * p.H * p.K * sizeof(float));
   pl.dp = boff(tc ? (size_t)pl.nc * p.H * 64 * 64 * es : 0);       // dP tiles, query-side -> key-side gradient kernel
   pl.dga = boff(tc ? (size_t)pl.nc * p.H * 64 * sizeof(float) : 0);  // dG partial sums, likewise
+  pl.z = boff(pl.delta && !tc ? (size_t)pl.nc * p.H * 64 * p.V * sizeof(float) : 0);
   const size_t slot_f32 = kda ? (size_t)pl.nc * p.H * 64 * p.K * sizeof(float) : 0;
   pl.kda_dag = boff(kda ? (size_t)pl.nc * p.H * 64 * 64 * es : 0);  // dAg tiles
   pl.kda_dqs = boff(slot_f32);                                      // gradients of the folded state-side operands
@@ -164,6 +166,8 @@ int launch_kkt_tc(const ChunkedCtx& c, cudaStream_t s);                         
 int launch_kda_prep(const ChunkedCtx& c, cudaStream_t s);                       // KDA: gate-folded operands, P, Ag
 int launch_kda_grads(const ChunkedCtx& c, const jla_bwd_io& io, char* scratch, cudaStream_t s);  // after the reverse pass
 int launch_sg_fwd(const ChunkedCtx& c, const jla_fwd_io& io, cudaStream_t s);
+int launch_split_fwd(const ChunkedCtx& c, const jla_fwd_io& io, cudaStream_t s);        // chunked_split.cu
+int launch_split_bwd_state(const ChunkedCtx& c, const jla_bwd_io& io, char* scratch, cudaStream_t s);
 int launch_sg_bwd(const ChunkedCtx& c, const jla_bwd_io& io, char* scratch, cudaStream_t s);
 int l2norm_fwd(const void* x, void* y, int dtype, long rows, int K, cudaStream_t stream);
 int launch_sg_fwd_tc(const ChunkedCtx& c, const jla_fwd_io& io, cudaStream_t s);

@@ -86,7 +86,8 @@ int chunked_fwd(const jla_problem& p, const jla_fwd_io& io, cudaStream_t stream)
     const int rc = launch_prep(c, stream);
     if (rc != JLA_OK) return rc;
   }
-  return use_tc_kernels(p) ? launch_sg_fwd_tc(c, io, stream) : launch_sg_fwd(c, io, stream);
+  if (use_tc_kernels(p)) return launch_sg_fwd_tc(c, io, stream);
+  return pl.save ? launch_split_fwd(c, io, stream) : launch_sg_fwd(c, io, stream);
 }
 
 int chunked_bwd(const jla_problem& p, const jla_bwd_io& io, cudaStream_t stream) {

@@ -1,5 +1,5 @@
-// Backward of the scalar-gate family, chunk-64: a reverse serial pass per (row, head) that carries dS in fp32
-// registers and emits dv, dVn and the per-chunk dS+, then a chunk-parallel kernel for dq, dk, dbeta, dg.
+// Backward of the scalar-gate family, chunk-64: a reverse serial pass that emits dv, dVn and the per-chunk dS+
+// (chunked_split.cu, chunked_bwd_state_tc.cu), then a chunk-parallel kernel for dq, dk, dbeta, dg.
 //
 //   dVn = scale P^T dO + (tail Gamma_r)(K dS+)       dW = Ag^T dVn = dV
 //   dS  = keep gamma dS+ + scale ((cin Gamma) Q)^T dO - ((cin Gamma) K)^T dW
@@ -20,232 +20,17 @@ namespace {
 
 struct BwdParams {
   const ChunkMeta* meta;
-  const int2* row_chunks;
   const float* gates;
   const unsigned char* runs;
   const void *q, *k, *v, *t0, *d_o, *h, *vn;
-  const float* d_final;
   const float* qk_tab;  // Q K^T and K Q^T per (chunk, key head) in fragment order (qk_table_kernel), or nullptr
-  void *dh, *dvn, *dv;
-  float* dh0;
+  const void *dh, *dvn, *dv;
   void *dq, *dk;          // tensor dtype, written directly when dq_acc == nullptr
   float *dq_acc, *dk_acc;  // [tokens, H, K] f32 otherwise
   float *dg, *dbeta;
   int H, Hk;
   float scale;
 };
-
-// ---------------------------------------------------------------------------------------------------------
-// reverse serial pass
-template <typename T, int K, int V, bool DELTA>
-struct BwdStateSmem {
-  static constexpr int LDK = K + 8, LDV = V + 8, LDC = 72;
-  static constexpr int kStageElems = 2 * 64 * LDK + 64 * LDV + (DELTA ? 64 * LDC : 0);
-  static constexpr int kStageBytes = kStageElems * 2 + 512 + 64;
-  // Without the delta rule only the 16-bit dS+ copy lives outside the stages: dv goes to global memory from the
-  // accumulators and the scale (cin Gamma) factor of the dS update is applied to the query fragments in registers.
-  static constexpr int kBytes = 2 * kStageBytes + (K * LDV + (DELTA ? 3 * 64 * LDV + 64 * LDC : 0)) * 2;
-};
-
-// (Two CTAs per SM for the Mamba-2 shape, as in the forward pass: 108 KB of shared memory and <= 128 registers each.)
-template <typename T, int K, int V, bool DELTA>
-__global__ void __launch_bounds__(256, (!DELTA && V == 64) ? 2 : 1) sg_bwd_state_kernel(BwdParams p) {
-  using L = BwdStateSmem<T, K, V, DELTA>;
-  constexpr int LDK = L::LDK, LDV = L::LDV, LDC = L::LDC;
-  constexpr int WR = K / 16, WC = 8 / WR, SNT = V / 8 / WC, ONT = V / 16;
-  const int row = blockIdx.x / p.H, h = blockIdx.x - row * p.H;
-  const int hk = h / (p.H / p.Hk);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  const int r0 = 16 * (warp & 3), c0 = (V / 2) * (warp >> 2);
-  const int sr0 = 16 * (warp % WR), sc0 = (V / WC) * (warp / WR);
-  const int2 rc = p.row_chunks[row];
-
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  auto stage_q = [&](int s) { return reinterpret_cast<T*>(smem_raw + s * L::kStageBytes); };
-  auto stage_k = [&](int s) { return stage_q(s) + 64 * LDK; };
-  auto stage_do = [&](int s) { return stage_k(s) + 64 * LDK; };
-  auto stage_t0 = [&](int s) { return stage_do(s) + 64 * LDV; };
-  auto stage_g = [&](int s) { return reinterpret_cast<float*>(smem_raw + s * L::kStageBytes + L::kStageElems * 2); };
-  auto stage_runs = [&](int s) { return reinterpret_cast<unsigned char*>(stage_g(s) + 128); };
-  T* dSb = reinterpret_cast<T*>(smem_raw + 2 * L::kStageBytes);
-  T* dVnb = dSb + K * LDV;
-  T* dOs = dVnb + 64 * LDV;
-  T* dWs = dOs + 64 * LDV;                       // DELTA only
-  T* AgT = dWs + 64 * LDV;                       // DELTA only
-
-  auto issue_load = [&](int ci, int s) {
-    const int c = rc.x + ci;
-    const ChunkMeta m = p.meta[c];
-    const T* q = static_cast<const T*>(p.q) + ((long)m.tok0 * p.Hk + hk) * K;
-    const T* k = static_cast<const T*>(p.k) + ((long)m.tok0 * p.Hk + hk) * K;
-    const T* d_o = static_cast<const T*>(p.d_o) + ((long)m.tok0 * p.H + h) * V;
-    load_tile_async<T, 64, K>(stage_q(s), LDK, q, (long)p.Hk * K, m.len, tid, 256);
-    load_tile_async<T, 64, K>(stage_k(s), LDK, k, (long)p.Hk * K, m.len, tid, 256);
-    load_tile_async<T, 64, V>(stage_do(s), LDV, d_o, (long)p.H * V, m.len, tid, 256);
-    if (DELTA) {
-      load_tile_async<T, 64, 64>(stage_t0(s), LDC, static_cast<const T*>(p.t0) + ((long)c * p.H + h) * 4096, 64, 64,
-                                 tid, 256);
-    }
-    if (tid < 32) cp_async16(stage_g(s) + tid * 4, p.gates + ((long)c * p.H + h) * 128 + tid * 4);
-    if (tid >= 32 && tid < 36) cp_async16(stage_runs(s) + (tid - 32) * 16, p.runs + (long)c * 64 + (tid - 32) * 16);
-    cp_async_commit();
-  };
-
-  float accD[SNT][4];
-  {
-    const float* df = p.d_final ? p.d_final + ((long)row * p.H + h) * K * V : nullptr;
-#pragma unroll
-    for (int nt = 0; nt < SNT; ++nt) {
-#pragma unroll
-      for (int hh = 0; hh < 2; ++hh) {
-        float2 x = make_float2(0.f, 0.f);
-        if (df) x = *reinterpret_cast<const float2*>(df + (long)(sr0 + g + 8 * hh) * V + sc0 + nt * 8 + 2 * t);
-        accD[nt][2 * hh] = x.x;
-        accD[nt][2 * hh + 1] = x.y;
-      }
-    }
-    store_acc<T, SNT>(dSb, LDV, sr0, sc0, accD, lane);
-  }
-  if (rc.y > 0) issue_load(rc.y - 1, 0);
-
-  for (int it = 0; it < rc.y; ++it) {
-    const int ci = rc.y - 1 - it;
-    const int s = it & 1;
-    const int c = rc.x + ci;
-    cp_async_wait<0>();
-    __syncthreads();  // S0
-    if (ci > 0) issue_load(ci - 1, s ^ 1);
-    const ChunkMeta m = p.meta[c];
-    const T* qS = stage_q(s);
-    const T* kS = stage_k(s);
-    const T* doS = stage_do(s);
-    const float* Gs = stage_g(s);
-    const float* betas = Gs + 64;
-    const unsigned char* runs = stage_runs(s);
-    const RowScalars rs0 = row_scalars(Gs, runs, m.flags, r0 + g);
-    const RowScalars rs1 = row_scalars(Gs, runs, m.flags, r0 + g + 8);
-
-    store_tile<T, V>(static_cast<T*>(p.dh) + ((long)c * p.H + h) * K * V, V, dSb, LDV, K, tid, 256);
-    if (!DELTA) {
-      // scale (cin Gamma) per token for the dS update, kept in the (unused) beta half of the gate vectors and
-      // applied to the query fragments (ordered before its readers by Sa)
-      if (tid < 64) stage_g(s)[64 + tid] = p.scale * row_scalars(Gs, runs, m.flags, tid).gam;
-    } else {  // dOs = scale (cin Gamma) dO; AgT[j][i] = Ag_ij
-      const int i = tid >> 2, j0 = (tid & 3) * (V / 4);
-      const float sg = p.scale * row_scalars(Gs, runs, m.flags, i).gam;
-#pragma unroll
-      for (int jj = 0; jj < V / 4; jj += 2) {
-        const float2 x = unpack2<T>(*reinterpret_cast<const uint32_t*>(doS + i * LDV + j0 + jj));
-        *reinterpret_cast<uint32_t*>(dOs + i * LDV + j0 + jj) = pack2<T>(x.x * sg, x.y * sg);
-      }
-      {
-        const T* t0S = stage_t0(s);
-        const int c16 = (tid & 3) * 16;
-        const float Gi = Gs[i];
-        const int runi = runs[i];
-#pragma unroll
-        for (int jj = 0; jj < 16; ++jj) {
-          const int j = c16 + jj;
-          const float a = to_f32(t0S[i * LDC + j]) * decay_ij(Gs, runs, i, j, Gi, runi) * betas[j];
-          AgT[j * LDC + i] = from_f32<T>(a);
-        }
-      }
-    }
-    // Pt[j][i] = scale (k_j . q_i) D_ij for this warp's 16 rows j and all 64 columns i
-    uint32_t pfrag[4][4];
-    {
-      float accP[8][4];
-      if (p.qk_tab) {  // K Q^T is shared by the value heads of the key head: this warp's fragments from the table
-        const float4* src = reinterpret_cast<const float4*>(p.qk_tab + ((long)c * p.Hk + hk) * kQkTabFloats + 4096) +
-                            (warp & 3) * 8 * 32 + lane;
-#pragma unroll
-        for (int nt = 0; nt < 8; ++nt) {
-          const float4 x = __ldg(src + nt * 32);
-          accP[nt][0] = x.x, accP[nt][1] = x.y, accP[nt][2] = x.z, accP[nt][3] = x.w;
-        }
-      } else {
-        zero_acc(accP);
-        warp_gemm<T, 8, K / 16, A_ROW, B_NK>(accP, kS + r0 * LDK, LDK, qS, LDK, lane);
-      }
-#pragma unroll
-      for (int nt = 0; nt < 8; ++nt) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int j = r0 + g + ((e >> 1) << 3), i = nt * 8 + 2 * t + (e & 1);
-          accP[nt][e] *= p.scale * decay_ij(Gs, runs, i, j, Gs[i], runs[i]);
-        }
-      }
-      acc_to_afrag<T, 4>(pfrag, accP);
-    }
-    // dVn = (tail Gamma_r)(K dS+) + scale P^T dO
-    float acc[ONT][4];
-    zero_acc(acc);
-    warp_gemm<T, ONT, K / 16, A_ROW, B_KN>(acc, kS + r0 * LDK, LDK, dSb + c0, LDV, lane);
-#pragma unroll
-    for (int nt = 0; nt < ONT; ++nt) {
-      acc[nt][0] *= rs0.gamr;
-      acc[nt][1] *= rs0.gamr;
-      acc[nt][2] *= rs1.gamr;
-      acc[nt][3] *= rs1.gamr;
-    }
-    warp_gemm_ra<T, ONT, 4, B_KN>(acc, pfrag, doS + c0, LDV, lane);
-    T* dv = static_cast<T*>(p.dv) + ((long)m.tok0 * p.H + h) * V;
-    if (DELTA) {
-      store_acc<T, ONT>(dVnb, LDV, r0, c0, acc, lane);
-    } else {  // dV = dVn, straight from the accumulators
-#pragma unroll
-      for (int nt = 0; nt < ONT; ++nt) {
-        const int col = c0 + nt * 8 + 2 * t;
-        if (r0 + g < m.len)
-          *reinterpret_cast<uint32_t*>(dv + (long)(r0 + g) * p.H * V + col) = pack2<T>(acc[nt][0], acc[nt][1]);
-        if (r0 + g + 8 < m.len)
-          *reinterpret_cast<uint32_t*>(dv + (long)(r0 + g + 8) * p.H * V + col) = pack2<T>(acc[nt][2], acc[nt][3]);
-      }
-    }
-    __syncthreads();  // Sa: dVnb, dOs, AgT complete; every warp is done reading dSb
-    if (DELTA) {
-      store_tile<T, V>(static_cast<T*>(p.dvn) + ((long)c * p.H + h) * 64 * V, V, dVnb, LDV, 64, tid, 256);
-      zero_acc(acc);
-      warp_gemm<T, ONT, 4, A_ROW, B_KN>(acc, AgT + r0 * LDC, LDC, dVnb + c0, LDV, lane);  // dW = Ag^T dVn
-#pragma unroll
-      for (int nt = 0; nt < ONT; ++nt) {
-        const int col = c0 + nt * 8 + 2 * t;
-        if (r0 + g < m.len)
-          *reinterpret_cast<uint32_t*>(dv + (long)(r0 + g) * p.H * V + col) = pack2<T>(acc[nt][0], acc[nt][1]);
-        if (r0 + g + 8 < m.len)
-          *reinterpret_cast<uint32_t*>(dv + (long)(r0 + g + 8) * p.H * V + col) = pack2<T>(acc[nt][2], acc[nt][3]);
-      }
-      store_acc<T, ONT>(dWs, LDV, r0, c0, acc, lane, -rs0.gam, -rs1.gam);
-      __syncthreads();  // Sb: dWs complete
-    }
-    // dS = keep gamma dS+ + Q^T (scale cin Gamma dO) - K^T (cin Gamma dW)
-    const float kg = keep_gamma(Gs, runs, m.flags);
-#pragma unroll
-    for (int nt = 0; nt < SNT; ++nt) {
-      accD[nt][0] *= kg;
-      accD[nt][1] *= kg;
-      accD[nt][2] *= kg;
-      accD[nt][3] *= kg;
-    }
-    if (DELTA) {
-      warp_gemm<T, SNT, 4, A_COL, B_KN>(accD, qS + sr0, LDK, dOs + sc0, LDV, lane);
-      warp_gemm<T, SNT, 4, A_COL, B_KN>(accD, kS + sr0, LDK, dWs + sc0, LDV, lane);
-    } else {
-      warp_gemm_scaled_a<T, SNT, 4, B_KN>(accD, qS + sr0, LDK, betas, doS + sc0, LDV, lane);
-    }
-    store_acc<T, SNT>(dSb, LDV, sr0, sc0, accD, lane);
-  }
-
-  if (p.dh0) {
-    float* f = p.dh0 + ((long)row * p.H + h) * K * V;
-#pragma unroll
-    for (int nt = 0; nt < SNT; ++nt) {
-      *reinterpret_cast<float2*>(f + (long)(sr0 + g) * V + sc0 + nt * 8 + 2 * t) = make_float2(accD[nt][0], accD[nt][1]);
-      *reinterpret_cast<float2*>(f + (long)(sr0 + g + 8) * V + sc0 + nt * 8 + 2 * t) =
-          make_float2(accD[nt][2], accD[nt][3]);
-    }
-  }
-}
 
 // ---------------------------------------------------------------------------------------------------------
 // chunk-parallel gradients
@@ -675,40 +460,28 @@ __global__ void __launch_bounds__(256, (!DELTA && V == 64) ? 2 : 1) sg_chunk_gra
 }
 
 template <typename T, int K, int V, bool DELTA>
-int launch_one(const BwdParams& bp, int rows_blocks, int chunk_blocks, bool legacy_grads, int head_walk, cudaStream_t s) {
+int launch_one(const BwdParams& bp, int chunk_blocks, int head_walk, cudaStream_t s) {
+  constexpr int smem = GradSmem<T, K, V, DELTA>::kBytes;
+  // the Mamba-2 shape with grouped heads: walks of 8, 4 or 2 heads per CTA (see the kernel)
+  auto* kern = sg_chunk_grads_kernel<T, K, V, DELTA, 1>;
+  if (!DELTA && V == 64 && K == 128 && head_walk == 8) kern = sg_chunk_grads_kernel<T, K, V, DELTA, (!DELTA && V == 64 && K == 128) ? 8 : 1>;
+  if (!DELTA && V == 64 && K == 128 && head_walk == 4) kern = sg_chunk_grads_kernel<T, K, V, DELTA, (!DELTA && V == 64 && K == 128) ? 4 : 1>;
+  if (!DELTA && V == 64 && K == 128 && head_walk == 2) kern = sg_chunk_grads_kernel<T, K, V, DELTA, (!DELTA && V == 64 && K == 128) ? 2 : 1>;
+  JLA_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
   {
-    auto* kern = sg_bwd_state_kernel<T, K, V, DELTA>;
-    constexpr int smem = BwdStateSmem<T, K, V, DELTA>::kBytes;
-    JLA_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    {
-      ProfScope ps(kProfSgBwdState, s);
-      kern<<<rows_blocks, 256, smem, s>>>(bp);
-    }
-    JLA_LAUNCH_OK();
+    ProfScope ps(kProfSgChunkGrads, s);
+    kern<<<chunk_blocks / head_walk, 256, smem, s>>>(bp);
   }
-  if (legacy_grads) {
-    constexpr int smem = GradSmem<T, K, V, DELTA>::kBytes;
-    // the Mamba-2 shape with grouped heads: walks of 8, 4 or 2 heads per CTA (see the kernel)
-    auto* kern = sg_chunk_grads_kernel<T, K, V, DELTA, 1>;
-    if (!DELTA && V == 64 && K == 128 && head_walk == 8) kern = sg_chunk_grads_kernel<T, K, V, DELTA, (!DELTA && V == 64 && K == 128) ? 8 : 1>;
-    if (!DELTA && V == 64 && K == 128 && head_walk == 4) kern = sg_chunk_grads_kernel<T, K, V, DELTA, (!DELTA && V == 64 && K == 128) ? 4 : 1>;
-    if (!DELTA && V == 64 && K == 128 && head_walk == 2) kern = sg_chunk_grads_kernel<T, K, V, DELTA, (!DELTA && V == 64 && K == 128) ? 2 : 1>;
-    JLA_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    {
-      ProfScope ps(kProfSgChunkGrads, s);
-      kern<<<chunk_blocks / head_walk, 256, smem, s>>>(bp);
-    }
-    JLA_LAUNCH_OK();
-  }
+  JLA_LAUNCH_OK();
   return JLA_OK;
 }
 
 template <typename T, bool DELTA>
-int launch_kv(const BwdParams& bp, int K, int V, int rb, int cb, bool legacy, int walk, cudaStream_t s) {
-  if (K == 128 && V == 128) return launch_one<T, 128, 128, DELTA>(bp, rb, cb, legacy, walk, s);
-  if (K == 128 && V == 64) return launch_one<T, 128, 64, DELTA>(bp, rb, cb, legacy, walk, s);
-  if (K == 64 && V == 128) return launch_one<T, 64, 128, DELTA>(bp, rb, cb, legacy, walk, s);
-  return launch_one<T, 64, 64, DELTA>(bp, rb, cb, legacy, walk, s);
+int launch_kv(const BwdParams& bp, int K, int V, int cb, int walk, cudaStream_t s) {
+  if (K == 128 && V == 128) return launch_one<T, 128, 128, DELTA>(bp, cb, walk, s);
+  if (K == 128 && V == 64) return launch_one<T, 128, 64, DELTA>(bp, cb, walk, s);
+  if (K == 64 && V == 128) return launch_one<T, 64, 128, DELTA>(bp, cb, walk, s);
+  return launch_one<T, 64, 64, DELTA>(bp, cb, walk, s);
 }
 
 }  // namespace
@@ -722,7 +495,6 @@ int launch_sg_bwd(const ChunkedCtx& c, const jla_bwd_io& io, char* scratch, cuda
   const bool direct = p.H == p.Hk && !pl.l2norm;
   BwdParams bp{};
   bp.meta = reinterpret_cast<const ChunkMeta*>(c.res + pl.meta);
-  bp.row_chunks = reinterpret_cast<const int2*>(c.res + pl.row_chunks);
   bp.gates = reinterpret_cast<const float*>(c.res + pl.gates);
   bp.runs = reinterpret_cast<const unsigned char*>(c.res + pl.runs);
   bp.q = c.q_eff;
@@ -732,12 +504,10 @@ int launch_sg_bwd(const ChunkedCtx& c, const jla_bwd_io& io, char* scratch, cuda
   bp.d_o = io.d_o;
   bp.h = c.res + pl.h;
   bp.vn = c.res + pl.vn;
-  bp.d_final = io.d_final;
   bp.qk_tab = shares_scores(p) ? reinterpret_cast<const float*>(c.res + pl.qk_tab) : nullptr;
   bp.dh = scratch + pl.dh;
   bp.dvn = scratch + pl.dvn;
   bp.dv = io.dv;
-  bp.dh0 = io.dh0;
   bp.dq = io.dq;
   bp.dk = io.dk;
   bp.dq_acc = direct ? nullptr : reinterpret_cast<float*>(scratch + pl.dq_acc);
@@ -747,21 +517,20 @@ int launch_sg_bwd(const ChunkedCtx& c, const jla_bwd_io& io, char* scratch, cuda
   bp.H = p.H;
   bp.Hk = p.Hk;
   bp.scale = p.scale;
-  const int rb = pl.rows * p.H, cb = pl.nc * p.H;
+  const int cb = pl.nc * p.H;
   const bool legacy = !use_tc_kernels(p);  // mma.sync chunk gradients (row-major residuals)
   // heads per CTA walk of the legacy gradient kernel (sums dq, dk over them in registers): the Mamba-2 shape with
   // grouped key heads only
   const int group = p.H / p.Hk;
   const int walk = (legacy && !direct && !pl.delta && p.K == 128 && p.V == 64) ? (group % 8 == 0 ? 8 : group % 4 == 0 ? 4 : group % 2 == 0 ? 2 : 1) : 1;
-  int rc;
-  if (!legacy) {
-    rc = launch_sg_bwd_state_tc(c, io, scratch, s);
-  } else if (p.dtype == JLA_DTYPE_BF16) {
-    rc = pl.delta ? launch_kv<__nv_bfloat16, true>(bp, p.K, p.V, rb, cb, legacy, walk, s)
-                  : launch_kv<__nv_bfloat16, false>(bp, p.K, p.V, rb, cb, legacy, walk, s);
-  } else {
-    rc = pl.delta ? launch_kv<__half, true>(bp, p.K, p.V, rb, cb, legacy, walk, s)
-                  : launch_kv<__half, false>(bp, p.K, p.V, rb, cb, legacy, walk, s);
+  int rc = legacy ? launch_split_bwd_state(c, io, scratch, s) : launch_sg_bwd_state_tc(c, io, scratch, s);
+  if (rc == JLA_OK && legacy) {
+    if (p.dtype == JLA_DTYPE_BF16) {
+      rc = pl.delta ? launch_kv<__nv_bfloat16, true>(bp, p.K, p.V, cb, walk, s)
+                    : launch_kv<__nv_bfloat16, false>(bp, p.K, p.V, cb, walk, s);
+    } else {
+      rc = pl.delta ? launch_kv<__half, true>(bp, p.K, p.V, cb, walk, s) : launch_kv<__half, false>(bp, p.K, p.V, cb, walk, s);
+    }
   }
   if (rc == JLA_OK && !legacy && (p.flags & JLA_FLAG_STATE_GRADS_ONLY)) return rc;
   if (rc == JLA_OK && !legacy) rc = kda ? launch_kda_grads(c, io, scratch, s) : launch_chunk_grads_tc(c, io, scratch, direct, s);

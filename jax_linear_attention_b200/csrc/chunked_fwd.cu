@@ -1,4 +1,5 @@
-// Forward of the scalar-gate family (simple GLA / DeltaNet / Gated DeltaNet), chunk-64, one CTA per
+// Forward of the scalar-gate family (simple GLA / DeltaNet / Gated DeltaNet) that keeps nothing for a backward (those
+// that do run chunked_split.cu), chunk-64, one CTA per
 // (row, head) walking the row's chunks with the fp32 state in registers.
 //
 // Per chunk (see chunked.cuh for the math): W = V - (cin Gamma)(K S); Vn = Ag W; P = (Q K^T) D;
@@ -24,7 +25,6 @@ struct FwdParams {
   const float* qk_tab;  // Q K^T per (chunk, key head) in fragment order (qk_table_kernel), or nullptr
   void* o;
   float* final_state;
-  void *h_out, *vn_out;  // residuals (nullptr when not saving)
   int H, Hk;
   float scale;
 };
@@ -124,9 +124,6 @@ __global__ void __launch_bounds__(256, (!DELTA && V == 64) ? 2 : 1) sg_fwd_kerne
     const RowScalars rs0 = row_scalars(Gs, runs, m.flags, r0 + g);
     const RowScalars rs1 = row_scalars(Gs, runs, m.flags, r0 + g + 8);
 
-    if (p.h_out) {
-      store_tile<T, V>(static_cast<T*>(p.h_out) + ((long)c * p.H + h) * K * V, V, Sb, LDV, K, tid, 256);
-    }
     if (DELTA) {
       // Ag = T0 * D * beta_j (row tid / 4, 16 columns per thread)
       const T* t0S = stage_t0(s);
@@ -212,9 +209,6 @@ __global__ void __launch_bounds__(256, (!DELTA && V == 64) ? 2 : 1) sg_fwd_kerne
     store_acc<T, ONT>(oS, LDO, r0, c0, accO, lane, p.scale, p.scale);
     __syncthreads();  // S4: every warp is done with Sb and the staging tile holds O
     store_tile<T, V>(static_cast<T*>(p.o) + ((long)m.tok0 * p.H + h) * V, (long)p.H * V, oS, LDO, m.len, tid, 256);
-    if (DELTA && p.vn_out) {
-      store_tile<T, V>(static_cast<T*>(p.vn_out) + ((long)c * p.H + h) * 64 * V, V, Vnb, LDV, 64, tid, 256);
-    }
     // S+ = keep gamma S + K^T (tail Gamma_r Vn)
     const float kg = keep_gamma(Gs, runs, m.flags);
 #pragma unroll
@@ -283,8 +277,6 @@ int launch_sg_fwd(const ChunkedCtx& c, const jla_fwd_io& io, cudaStream_t s) {
   fp.qk_tab = shares_scores(p) ? reinterpret_cast<const float*>(c.res + pl.qk_tab) : nullptr;
   fp.o = io.o;
   fp.final_state = io.final_state;
-  fp.h_out = pl.save ? c.res + pl.h : nullptr;
-  fp.vn_out = pl.save && pl.delta ? c.res + pl.vn : nullptr;
   fp.H = p.H;
   fp.Hk = p.Hk;
   fp.scale = p.scale;

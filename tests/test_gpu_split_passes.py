@@ -1,0 +1,29 @@
+"""The split training kernels (head sizes other than K = V = 128) on both sides of their size rules: value blocks of 32 and
+64 columns (few and many chains), walks of one and of eight heads, ragged last chunks, documents inside chunks, initial
+and final states. Reference: the fp32 token scan on the same 16-bit tensors, itself held to the float64 oracle. The error
+is that of 16-bit operands and outputs (bf16: 2^-9 per rounding, a few roundings in a row; f16 an eighth of that)."""
+
+import pytest
+import torch
+
+from oracle.cases import make_case
+from tests._util import compare, run_cuda
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("kind,B,T,H,Hk,K,V,dtype", [
+    ("simple_gla", 10, 130, 64, 1, 128, 64, "bfloat16"),   # 640 chains, walks of eight heads
+    ("simple_gla", 1, 65, 8, 1, 128, 64, "float16"),       # few chains, one head a CTA
+    ("simple_gla", 2, 63, 4, 2, 64, 128, "bfloat16"),
+    ("gated_deltanet", 20, 129, 32, 16, 64, 64, "bfloat16"),  # 640 chains
+    ("gated_deltanet", 2, 1, 2, 1, 64, 64, "float16"),
+    ("deltanet", 3, 191, 4, 4, 128, 64, "float16"),
+    ("gated_deltanet", 10, 70, 32, 32, 64, 128, "bfloat16"),
+    ("gated_deltanet", 1, 64, 40, 5, 128, 64, "bfloat16"),
+])
+def test_split_passes_match_the_scan(kind, B, T, H, Hk, K, V, dtype):
+    case = make_case(kind, B=B, T=T, H=H, Hk=Hk, K=K, V=V, seed=B + T, dtype=dtype, docs="mixed" if T > 8 else None, h0=True)
+    want = run_cuda(kind, case, scale=case["meta"]["scale"], dtype=dtype, precision="highest")
+    got = run_cuda(kind, case, scale=case["meta"]["scale"], dtype=dtype)
+    compare(got, want, {"bfloat16": 1e-2, "float16": 2e-3}[dtype], f"{kind} B{B} T{T} H{H} K{K} V{V}")
