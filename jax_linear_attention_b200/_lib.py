@@ -8,6 +8,8 @@ from __future__ import annotations
 import ctypes as C
 import os
 
+import torch
+
 HERE = os.path.dirname(os.path.abspath(__file__))
 # The in-tree build's output; JLA_B200_LIB names another build of the same library (e.g. the CMake build's).
 LIB_PATH = os.environ.get("JLA_B200_LIB") or os.path.join(HERE, "libjla_b200.so")
@@ -84,12 +86,41 @@ def load() -> C.CDLL:
     lib.jla_gdn2_inputs_fwd.argtypes = [C.c_int, C.c_int64, C.c_int64] + [C.c_void_p] * 7
     lib.jla_gdn2_inputs_bwd.restype = C.c_int
     lib.jla_gdn2_inputs_bwd.argtypes = [C.c_int, C.c_int64, C.c_int64] + [C.c_void_p] * 11
+    int_, i64, ptr, f32 = C.c_int, C.c_int64, C.c_void_p, C.c_float
+    for name, types in {  # typed, so that callers pass plain integers (data pointers) and None
+        "jla_short_conv_fwd": [int_] * 7 + [ptr] * 7, "jla_short_conv_bwd": [int_] * 7 + [ptr] * 11,
+        "jla_gate_prologue_fwd": [int_, i64, int_, int_] + [ptr] * 4 + [int_] + [ptr] * 3,
+        "jla_gate_prologue_bwd": [int_, i64, int_, int_] + [ptr] * 4 + [int_] + [ptr] * 7,
+        "jla_gated_rmsnorm_fwd": [int_, i64, int_, int_] + [ptr] * 3 + [f32, int_, int_] + [ptr] * 2,
+        "jla_gated_rmsnorm_bwd": [int_, i64, int_, int_] + [ptr] * 3 + [f32, int_, int_] + [ptr] * 5,
+        "jla_ssd_inputs_fwd": [int_, i64, int_, int_] + [ptr] * 6, "jla_ssd_inputs_bwd": [int_, i64, int_, int_] + [ptr] * 9,
+        "jla_ssd_output_fwd": [int_, i64, int_, int_] + [ptr] * 5, "jla_ssd_output_bwd": [int_, i64, int_, int_] + [ptr] * 6,
+        "jla_ssd_layer_bwd": [int_, i64, int_, int_] + [ptr] * 12,
+        "jla_ssd_step": [C.POINTER(Problem)] + [ptr] * 6,
+    }.items():
+        fn = getattr(lib, name)
+        fn.restype, fn.argtypes = C.c_int, types
     lib.jla_device_status.restype = C.c_int
     lib.jla_device_status.argtypes = [C.POINTER(C.c_int), C.c_void_p]
     lib.jla_selftest_bounded_wait.restype = C.c_int
     lib.jla_selftest_bounded_wait.argtypes = [C.c_uint32, C.c_void_p]
     _lib = lib
     return lib
+
+
+def launch(name: str, device, *args) -> None:
+    """``name(*args, stream)`` on ``device``'s current stream, with ``device`` current; raises on an error status. The host
+    cost of a call is what bounds the small ones, so the device is only switched where it is another one."""
+    fn = getattr(_lib or load(), name)
+    index = device.index
+    stream = torch._C._cuda_getCurrentRawStream(index)
+    if index == torch._C._cuda_getDevice():
+        rc = fn(*args, stream)
+    else:
+        with torch.cuda.device(device):
+            rc = fn(*args, stream)
+    if rc != OK:
+        check(rc, name)
 
 
 def device_status(stream: int | None = None) -> int:

@@ -21,14 +21,11 @@ _DTYPES = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}
 
 
 def _ptr(t):
-    return C.c_void_p(None if t is None else t.data_ptr())
+    return None if t is None else t.data_ptr()
 
 
 def _call(name, x, *args):
-    lib = _lib.load()
-    stream = torch.cuda.current_stream(x.device).cuda_stream
-    with torch.cuda.device(x.device):
-        _lib.check(getattr(lib, name)(*args, C.c_void_p(stream)), name)
+    _lib.launch(name, x.device, *args)
 
 
 class _ShortConv(torch.autograd.Function):
@@ -63,11 +60,11 @@ class _ShortConv(torch.autograd.Function):
 def _final_state(x, state, segment_ids, width: int):
     """The last ``width - 1`` inputs, zeroed where they precede the last token's document (conv.py:190-210)."""
     B, T, Cn = x.shape
-    if state is None:
-        state = x.new_zeros(B, width - 1, Cn)
     if T >= width - 1:
         tail = x[:, T - (width - 1):]
     else:
+        if state is None:
+            state = x.new_zeros(B, width - 1, Cn)
         tail = torch.cat([state[:, T:], x], dim=1)
     if segment_ids is not None and width > 1:
         seg = segment_ids
@@ -75,7 +72,7 @@ def _final_state(x, state, segment_ids, width: int):
             seg_tail = seg[:, T - (width - 1):]
         else:
             seg_tail = torch.cat([seg[:, :1].expand(B, width - 1 - T), seg], dim=1)
-        tail = torch.where((seg_tail == seg[:, -1:])[..., None], tail, torch.zeros((), dtype=x.dtype, device=x.device))
+        tail = tail.masked_fill((seg_tail != seg[:, -1:])[..., None], 0)
     return tail
 
 

@@ -19,14 +19,11 @@ _DTYPES = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}
 
 
 def _call(name: str, a: torch.Tensor, *args):
-    lib = _lib.load()
-    stream = torch.cuda.current_stream(a.device).cuda_stream
-    with torch.cuda.device(a.device):
-        _lib.check(getattr(lib, name)(*args, C.c_void_p(stream)), name)
+    _lib.launch(name, a.device, *args)
 
 
 def _ptr(t):
-    return C.c_void_p(None if t is None else t.data_ptr())
+    return None if t is None else t.data_ptr()
 
 
 class _GatePrologue(torch.autograd.Function):
@@ -37,7 +34,7 @@ class _GatePrologue(torch.autograd.Function):
         tokens = a.shape[0] * a.shape[1]
         g = torch.empty(a.shape, dtype=torch.float32, device=a.device)
         beta = None if b is None else torch.empty(b.shape, dtype=torch.float32, device=a.device)
-        _call("jla_gate_prologue_fwd", a, _DTYPES[a.dtype], C.c_int64(tokens), heads, width, _ptr(a), _ptr(a_log),
+        _call("jla_gate_prologue_fwd", a, _DTYPES[a.dtype], tokens, heads, width, _ptr(a), _ptr(a_log),
               _ptr(dt_bias), _ptr(b), int(allow_neg), _ptr(g), _ptr(beta))
         ctx.save_for_backward(a, a_log, dt_bias, b)
         ctx.allow_neg = allow_neg
@@ -57,7 +54,7 @@ class _GatePrologue(torch.autograd.Function):
         db = None if b is None else torch.empty_like(b)
         da_log = torch.empty_like(a_log)
         ddt_bias = torch.empty_like(dt_bias)
-        _call("jla_gate_prologue_bwd", a, _DTYPES[a.dtype], C.c_int64(tokens), heads, width, _ptr(a), _ptr(a_log),
+        _call("jla_gate_prologue_bwd", a, _DTYPES[a.dtype], tokens, heads, width, _ptr(a), _ptr(a_log),
               _ptr(dt_bias), _ptr(b), int(ctx.allow_neg), _ptr(dg), _ptr(None if b is None else dbeta), _ptr(da),
               _ptr(db), _ptr(da_log), _ptr(ddt_bias))
         return da, da_log, ddt_bias, db, None

@@ -19,14 +19,11 @@ _DTYPES = {torch.bfloat16: 0, torch.float16: 1, torch.float32: 2}
 
 
 def _call(name, x, *args):
-    lib = _lib.load()
-    stream = torch.cuda.current_stream(x.device).cuda_stream
-    with torch.cuda.device(x.device):
-        _lib.check(getattr(lib, name)(*args, C.c_void_p(stream)), name)
+    _lib.launch(name, x.device, *args)
 
 
 def _ptr(t):
-    return C.c_void_p(t.data_ptr())
+    return t.data_ptr()
 
 
 class _GatedRMSNorm(torch.autograd.Function):
@@ -35,8 +32,8 @@ class _GatedRMSNorm(torch.autograd.Function):
         dim = x.shape[-1]
         rows = x.numel() // dim
         y = torch.empty_like(x)
-        _call("jla_gated_rmsnorm_fwd", x, _DTYPES[x.dtype], C.c_int64(rows), dim, group, _ptr(x), _ptr(z), _ptr(weight),
-              C.c_float(eps), int(sigmoid_gate), int(norm_before_gate), _ptr(y))
+        _call("jla_gated_rmsnorm_fwd", x, _DTYPES[x.dtype], rows, dim, group, _ptr(x), _ptr(z), _ptr(weight),
+              eps, int(sigmoid_gate), int(norm_before_gate), _ptr(y))
         ctx.save_for_backward(x, z, weight)
         ctx.cfg = (eps, sigmoid_gate, norm_before_gate, group)
         return y
@@ -50,8 +47,8 @@ class _GatedRMSNorm(torch.autograd.Function):
         rows = x.numel() // dim
         dy = dy.contiguous()
         dx, dz, dw = torch.empty_like(x), torch.empty_like(z), torch.empty_like(weight)
-        _call("jla_gated_rmsnorm_bwd", x, _DTYPES[x.dtype], C.c_int64(rows), dim, group, _ptr(x), _ptr(z), _ptr(weight),
-              C.c_float(eps), int(sigmoid_gate), int(norm_before_gate), _ptr(dy), _ptr(dx), _ptr(dz), _ptr(dw))
+        _call("jla_gated_rmsnorm_bwd", x, _DTYPES[x.dtype], rows, dim, group, _ptr(x), _ptr(z), _ptr(weight),
+              eps, int(sigmoid_gate), int(norm_before_gate), _ptr(dy), _ptr(dx), _ptr(dz), _ptr(dw))
         return dx, dz, dw, None, None, None, None
 
 

@@ -73,34 +73,27 @@ def _step(x, dt, a, b, c, d, segment_ids, initial_state, output_final_state, chu
     batch, _, heads, width = x.shape
     groups, n = b.shape[2:]
     options = dict(initial_state=initial_state, segment_ids=segment_ids, chunk_size=chunk_size, precision=precision)
+    b = ops.cuda.cast(b, c.dtype)
     if (c.dtype != x.dtype or n not in (64, 128, 256) or width % 64 or precision == "chunked"
             or (d is not None and d.shape != (heads,))
-            or ops.cuda.unsupported_reason("simple_gla", c, b.to(c.dtype), x, (dt,), options) is not None):
+            or ops.cuda._reason("simple_gla", c, b, x, (dt,), options) is not None):
         return None
-    p = ops.cuda._problem("simple_gla", x.dtype, batch, 1, heads, groups, n, width, 0, 1.0, 0, precision)
-    dev = x.device
-    keep = [t if t is None else t.to(device=dev, dtype=td).contiguous() for t, td in
-            ((c, c.dtype), (b, c.dtype), (x, x.dtype), (initial_state, torch.float32), (dt, torch.float32),
-             (a, torch.float32), (d, torch.float32))]
-    p.q, p.k, p.v, p.h0, dt_ptr, a_ptr, d_ptr = (None if t is None else t.data_ptr() for t in keep)
-    y = torch.empty_like(keep[2])
-    final = torch.empty(batch, heads, n, width, dtype=torch.float32, device=dev) if output_final_state else None
-    stream = torch.cuda.current_stream(dev).cuda_stream
-    with torch.cuda.device(dev):
-        _lib.check(_lib.load().jla_ssd_step(C.byref(p), C.c_void_p(dt_ptr), C.c_void_p(a_ptr), C.c_void_p(d_ptr),
-                                            C.c_void_p(y.data_ptr()),
-                                            C.c_void_p(None if final is None else final.data_ptr()),
-                                            C.c_void_p(stream)), "ssd step")
+    dev, f32 = x.device, torch.float32
+    c, b, x = (ops.cuda.cast(t, c.dtype, dev) for t in (c, b, x))
+    dt, a, d, initial_state = (ops.cuda.cast(t, f32, dev) for t in (dt, a, d, initial_state))
+    p = ops.cuda._problem("simple_gla", x.dtype, batch, 1, heads, groups, n, width, 0, 1.0, 0, precision,
+                          c.data_ptr(), b.data_ptr(), x.data_ptr(), None, None,
+                          None if initial_state is None else initial_state.data_ptr())
+    y = torch.empty_like(x)
+    final = torch.empty(batch, heads, n, width, dtype=f32, device=dev) if output_final_state else None
+    _lib.launch("jla_ssd_step", dev, p, dt.data_ptr(), a.data_ptr(), None if d is None else d.data_ptr(), y.data_ptr(),
+                None if final is None else final.data_ptr())
     return y, final
 
 
 def _glue_call(name: str, x: torch.Tensor, *args):
-    lib = _lib.load()
-    tokens, heads, p = x.shape[0] * x.shape[1], x.shape[2], x.shape[3]
-    stream = torch.cuda.current_stream(x.device).cuda_stream
-    ptrs = [C.c_void_p(t.data_ptr()) for t in args]
-    with torch.cuda.device(x.device):
-        _lib.check(getattr(lib, name)(_DTYPES[x.dtype], C.c_int64(tokens), heads, p, *ptrs, C.c_void_p(stream)), name)
+    batch, seq_len, heads, width = x.shape
+    _lib.launch(name, x.device, _DTYPES[x.dtype], batch * seq_len, heads, width, *(t.data_ptr() for t in args))
 
 
 class _SsdInputs(torch.autograd.Function):

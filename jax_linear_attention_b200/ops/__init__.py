@@ -71,7 +71,7 @@ def linear_attention(kind: str, q, k, v, *, impl: str = "auto", **inputs: Any):
         raise ValueError(f"unknown linear-attention kind {kind!r}; expected one of {sorted(KINDS)}")
     _, gate_names = KINDS[kind]
     missing = [name for name in gate_names if inputs.get(name) is None]
-    extra = sorted(name for name in _GATE_NAMES - set(gate_names) if inputs.get(name) is not None)
+    extra = sorted(name for name in _GATE_NAMES if name not in gate_names and inputs.get(name) is not None)
     if missing or extra:
         raise ValueError(f"{kind} takes gates {gate_names}; missing {missing}, unexpected {extra}")
     gates = [inputs.pop(name) for name in gate_names]
@@ -82,8 +82,11 @@ def linear_attention(kind: str, q, k, v, *, impl: str = "auto", **inputs: Any):
         if entry is None:
             continue
         fn, supports, auto_eligible = entry
-        if impl == "auto" and not (auto_eligible and supports(q, k, v, *gates, **options)):
-            continue
+        if impl == "auto":
+            if not (auto_eligible and supports(q, k, v, *gates, **options)):
+                continue
+            if fn is cuda.FUNCTIONS[kind] and supports is cuda.SUPPORTS[kind]:
+                return cuda.run_checked(kind, q, k, v, *gates, **options)
         return fn(q, k, v, *gates, **options)
     if impl == "auto":  # surface the kernels' reason instead of a bare "nothing accepts this call"
         why = cuda.unsupported_reason(kind, q, k, v, tuple(gates), options)
