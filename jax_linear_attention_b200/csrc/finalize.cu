@@ -91,9 +91,45 @@ __global__ void finalize_key_grad_kernel(const float* __restrict__ acc, const T*
   }
 }
 
-// y = x * rsqrt(sum x^2 + 1e-6), fp32 math, rounded to the tensor dtype (reference.py:65-69). One warp per row.
+// y = x * rsqrt(sum x^2 + 1e-6), fp32 math, rounded to the tensor dtype (reference.py:65-69). HBM-bound: a row of K
+// channels belongs to K / VEC adjacent lanes with one 16-byte load each, and every lane group has ROWS rows' loads in
+// flight before the first sum (a warp per row with 2-byte loads took 7.8 us for the 10 MB of 5003 x 8 x 128).
+template <typename T, int ROWS>
+__global__ void __launch_bounds__(256) l2norm_fwd_kernel(const T* __restrict__ x, T* __restrict__ y, long rows, int K) {
+  constexpr int VEC = 16 / (int)sizeof(T);
+  const int lanes = K / VEC;  // a power of two <= 32 (checked by the launcher)
+  const int groups = 256 / lanes;
+  const int lg = threadIdx.x / lanes, ln = threadIdx.x - lg * lanes;
+  const long r0 = (long)blockIdx.x * groups * ROWS + lg;
+  uint4 raw[ROWS];
+#pragma unroll
+  for (int i = 0; i < ROWS; ++i) {
+    const long r = r0 + (long)i * groups;
+    raw[i] = r < rows ? reinterpret_cast<const uint4*>(x + r * K)[ln] : make_uint4(0, 0, 0, 0);
+  }
+#pragma unroll
+  for (int i = 0; i < ROWS; ++i) {
+    const T* e = reinterpret_cast<const T*>(&raw[i]);
+    float v[VEC], sumsq = 0.f;
+#pragma unroll
+    for (int c = 0; c < VEC; ++c) {
+      v[c] = to_f32(e[c]);
+      sumsq += v[c] * v[c];
+    }
+    for (int off = lanes >> 1; off > 0; off >>= 1) sumsq += __shfl_xor_sync(0xffffffffu, sumsq, off);
+    const float inv = rsqrtf(sumsq + 1e-6f);
+    uint4 out;
+    T* o = reinterpret_cast<T*>(&out);
+#pragma unroll
+    for (int c = 0; c < VEC; ++c) o[c] = from_f32<T>(v[c] * inv);
+    const long r = r0 + (long)i * groups;
+    if (r < rows) reinterpret_cast<uint4*>(y + r * K)[ln] = out;
+  }
+}
+
+// The same for rows that are not whole groups of 16 aligned bytes: one warp per row, an element at a time.
 template <typename T>
-__global__ void l2norm_fwd_kernel(const T* __restrict__ x, T* __restrict__ y, long rows, int K) {
+__global__ void __launch_bounds__(256) l2norm_rows_kernel(const T* __restrict__ x, T* __restrict__ y, long rows, int K) {
   const long row = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= rows) return;
   const int lane = threadIdx.x & 31;
@@ -132,12 +168,18 @@ int finalize_t(const float* acc, const void* raw, void* out, long rows, int H, i
 template <typename T>
 int l2norm_t(const void* x, void* y, long rows, int K, cudaStream_t stream) {
   if (rows == 0) return JLA_OK;
-  const int warps = 8;
-  const long blocks = (rows + warps - 1) / warps;
-  {
-    ProfScope ps(kProfL2Norm, stream);
-    l2norm_fwd_kernel<T><<<(unsigned)blocks, warps * 32, 0, stream>>>(static_cast<const T*>(x), static_cast<T*>(y),
-                                                                       rows, K);
+  constexpr int kRows = 4;
+  const int lanes = K * (int)sizeof(T) / 16;
+  const bool vec = K * sizeof(T) % 16 == 0 && lanes <= 32 && (lanes & (lanes - 1)) == 0 &&
+                   ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0;
+  ProfScope ps(kProfL2Norm, stream);
+  if (vec) {
+    const long per = 256 / lanes * kRows;
+    l2norm_fwd_kernel<T, kRows><<<(unsigned)((rows + per - 1) / per), 256, 0, stream>>>(static_cast<const T*>(x),
+                                                                                        static_cast<T*>(y), rows, K);
+  } else {
+    l2norm_rows_kernel<T><<<(unsigned)((rows + 7) / 8), 256, 0, stream>>>(static_cast<const T*>(x), static_cast<T*>(y),
+                                                                         rows, K);
   }
   JLA_LAUNCH_OK();
   return JLA_OK;
