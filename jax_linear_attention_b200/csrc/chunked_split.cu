@@ -4,8 +4,8 @@
 //             S+ = keep gamma S + K^T (tail Gamma_r Vn), leaving h (the state entering every chunk) and Vn behind;
 //             then all outputs at once: O = scale [(cin Gamma)(Q h) + ((Q K^T) D) Vn]
 //   backward  all Z = scale P^T dO at once (delta rule); the reverse state pass dVn = (tail Gamma_r)(K dS+) + Z;
-//             dW = dV = Ag^T dVn; dS = keep gamma dS+ + Q^T (scale cin Gamma dO) - K^T (cin Gamma dW), leaving dh;
-//             without the delta rule then all dV = (tail Gamma_r)(K dh) + scale P^T dO at once
+//             dW = dV = Ag^T dVn; dS = keep gamma dS+ + Q^T (scale cin Gamma dO) - K^T (cin Gamma dW), leaving dh
+//             (without the delta rule dV needs no state of its own and is the gradient kernel's, chunked_bwd.cu)
 //
 // A state pass walks a row's chunks, so its time is the number of chunks times the length of one chunk's chain of
 // dependent products; the forms that also computed scores and outputs inside the walk took 6.8 us a chunk (24 chains of
@@ -14,6 +14,10 @@
 // barrier without, on four warps; the value columns of a state are independent, so a call with few chains runs them in
 // blocks of VB. What is read back for the outputs (h, Vn) the backward keeps anyway. Forwards that keep nothing stay on
 // the fused kernel (chunked_fwd.cu), which needs no scratch for h.
+//
+// Measured: the walks of the d = 64 shape 23 + 33 us (fused 109 + 119), of the Mamba-2 shape 175 + 170 us and its outputs
+// 150 us (fused 439 + 436); what bounds them now is the latency of a chunk's loads, barriers and products at one to four
+// CTAs of four warps an SM.
 //
 // Rounding is that of the fused kernels: 16-bit operands, fp32 accumulation, the carried state in fp32, Z in fp32.
 #include "chunked.cuh"
@@ -49,7 +53,7 @@ struct StateSmem {
   static constexpr bool kQ = BWD, kK = DELTA || !BWD;  // tiles a stage holds
   static constexpr int kStageElems = ((kQ ? 1 : 0) + (kK ? 1 : 0)) * 64 * LDK + 64 * LDV + (DELTA ? 64 * LDC : 0);
   static constexpr int kStageBytes = kStageElems * 2 + 512 + 64;  // + gates (128 f32) + runs (64 u8)
-  static constexpr int kTiles = K * LDV + (DELTA ? 3 * 64 * LDV : 0);
+  static constexpr int kTiles = DELTA ? K * LDV + 3 * 64 * LDV : 0;
   static constexpr int kBytes = 2 * kStageBytes + kTiles * 2;
 };
 
@@ -79,9 +83,8 @@ __global__ void __launch_bounds__(NT) state_kernel(StateParams p) {
   T* A2 = A1 + 64 * LDV;   // Vn, dVn
   T* A3 = A2 + 64 * LDV;   // (tail Gamma_r) Vn
 
-  auto issue_load = [&](int ci, int s) {
+  auto issue_load = [&](int ci, int s, const ChunkMeta& m) {
     const int c = rc.x + ci;
-    const ChunkMeta m = p.meta[c];
     const long key = ((long)m.tok0 * p.Hk + hk) * K;
     if (L::kQ) load_tile_async<T, 64, K>(stage_q(s), LDK, static_cast<const T*>(p.q) + key, (long)p.Hk * K, m.len, tid, NT);
     if (L::kK) load_tile_async<T, 64, K>(stage_k(s), LDK, static_cast<const T*>(p.k) + key, (long)p.Hk * K, m.len, tid, NT);
@@ -118,12 +121,16 @@ __global__ void __launch_bounds__(NT) state_kernel(StateParams p) {
         acc[mt][nt][2 * hh] = x.x, acc[mt][nt][2 * hh + 1] = x.y;
       }
     }
-    store_acc<T, NTV>(Sb, LDV, sr0 + 16 * mt, 0, acc[mt], lane);
+    if (DELTA) store_acc<T, NTV>(Sb, LDV, sr0 + 16 * mt, 0, acc[mt], lane);
   }
   const int n = rc.y;
   auto chunk_at = [&](int it) { return BWD ? n - 1 - it : it; };
+  // table entries of this chunk, of the next one (whose loads it addresses) and of the one after, read a chunk ahead
+  ChunkMeta m{}, m1{}, m2{};
+  if (n > 0) m1 = p.meta[rc.x + chunk_at(0)];
+  if (n > 1) m2 = p.meta[rc.x + chunk_at(1)];
   if (n > 0) {
-    issue_load(chunk_at(0), 0);
+    issue_load(chunk_at(0), 0, m1);
     if (BWD && DELTA) load_z(chunk_at(0));
   }
 
@@ -131,8 +138,9 @@ __global__ void __launch_bounds__(NT) state_kernel(StateParams p) {
     const int s = it & 1, c = rc.x + chunk_at(it);
     cp_async_wait<0>();
     __syncthreads();  // the stage has landed, Sb holds the state, the other stage is free
-    if (it + 1 < n) issue_load(chunk_at(it + 1), s ^ 1);
-    const ChunkMeta m = p.meta[c];
+    m = m1, m1 = m2;
+    if (it + 1 < n) issue_load(chunk_at(it + 1), s ^ 1, m1);
+    if (it + 2 < n) m2 = p.meta[rc.x + chunk_at(it + 2)];
     const float* Gs = stage_g(s);
     const unsigned char* runs = stage_runs(s);
     const float kg = keep_gamma(Gs, runs, m.flags);
@@ -191,10 +199,11 @@ __global__ void __launch_bounds__(NT) state_kernel(StateParams p) {
       }
     } else {
       __syncthreads();
-      // a warp's rows of Sb are its own here: no other warp reads them
-      const int rows = 16 * MT;
-      store_tile<T, VB>(hout + (long)sr0 * p.V, p.V, Sb + sr0 * LDV, LDV, rows, lane, 32);
-      __syncwarp();
+      // straight from the accumulators: a 16-bit copy in shared memory would leave room for one CTA less on an SM
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt) {
+        store_acc<T, NTV>(hout, p.V, sr0 + 16 * mt, 0, acc[mt], lane);
+      }
     }
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt) {
@@ -221,7 +230,7 @@ __global__ void __launch_bounds__(NT) state_kernel(StateParams p) {
       }
     }
 #pragma unroll
-    for (int mt = 0; mt < MT; ++mt) store_acc<T, NTV>(Sb, LDV, sr0 + 16 * mt, 0, acc[mt], lane);
+    for (int mt = 0; mt < MT && DELTA; ++mt) store_acc<T, NTV>(Sb, LDV, sr0 + 16 * mt, 0, acc[mt], lane);
   }
 
   if (p.last) {
@@ -240,16 +249,15 @@ __global__ void __launch_bounds__(NT) state_kernel(StateParams p) {
 
 // ---------------------------------------------------------------------------------------------------------
 // everything that is not serial: per chunk and head (row r, column c of the score tile are tokens of the chunk)
-//   kOut : y = o  = scale [(cin Gamma_r)(q_r h) + sum_{c <= r} (q_r . k_c) D_rc x_c],        x = Vn (v without the delta rule)
-//   kGrad: y = dv = (tail Gamma_r)(k_r dh) + sum_{c >= r} scale (k_r . q_c) D_cr x_c,        x = dO
-//   kZ   : y = Z  = the second term of kGrad in fp32
-enum { kOut = 0, kGrad = 1, kZ = 2 };
+//   kOut: y = o = scale [(cin Gamma_r)(q_r h) + sum_{c <= r} (q_r . k_c) D_rc x_c],   x = Vn (v without the delta rule)
+//   kZ  : y = Z = sum_{c >= r} scale (k_r . q_c) D_cr x_c in fp32,                    x = dO
+enum { kOut = 0, kZ = 1 };
 
 struct TokenParams {
   const ChunkMeta* meta;
   const float* gates;
   const unsigned char* runs;
-  const void *a, *b;  // rows and columns of the scores: q, k (kOut) or k, q, [tokens, Hk, K]
+  const void *a, *b;  // rows and columns of the scores: q, k (kOut) or k, q (kZ), [tokens, Hk, K]
   const void* x;      // [tokens, H, V], or [chunk slot, H, 64, V] where x_slots
   const void* h;      // [chunk slot, H, K, V]
   void* y;            // [tokens, H, V] in the tensors' dtype; kZ: [chunk slot, H, 64, V] f32
@@ -261,15 +269,15 @@ template <typename T, int K, int V, int MODE, int NH>
 struct TokenSmem {
   static constexpr int LDK = K + 8, LDV = V + 8;
   static constexpr int kStageElems = 64 * LDV + (MODE == kZ ? 0 : K * LDV);
-  static constexpr int kStages = NH > 1 ? 2 : 1;
   static constexpr int kOutElems = MODE == kZ ? 0 : 64 * LDV;
-  static constexpr int kBytes = (2 * 64 * LDK + kStages * kStageElems + kOutElems) * 2 + kStages * 256 + 64;
+  static constexpr int kBytes = (2 * 64 * LDK + kStageElems + kOutElems) * 2 + 2 * 256 + 64;
+  static_assert(NH == 1 || kStageElems <= 2 * 64 * LDK, "the second stage lies over the key tiles");
 };
 
 // Four warps, 16 rows each. NH > 1: the CTA walks NH adjacent value heads of one key head, for which the raw scores are
-// the same products: they stay in registers, and the next head's tiles are on their way while one is worked on.
+// the same products: they stay in registers (as do a warp's rows of the state product's left operand), and the next head's tiles are on their way while one is worked on.
 template <typename T, int K, int V, int MODE, int NH>
-__global__ void __launch_bounds__(NT) token_kernel(TokenParams p) {
+__global__ void __launch_bounds__(NT, NH > 1 ? 3 : 1) token_kernel(TokenParams p) {
   using L = TokenSmem<T, K, V, MODE, NH>;
   constexpr int LDK = L::LDK, LDV = L::LDV, NTV = V / 8;
   const int hgs = p.H / NH;
@@ -285,11 +293,13 @@ __global__ void __launch_bounds__(NT) token_kernel(TokenParams p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T* aS = reinterpret_cast<T*>(smem_raw);
   T* bS = aS + 64 * LDK;
-  auto stage_x = [&](int s) { return bS + 64 * LDK + s * L::kStageElems; };
+  // NH > 1: once the scores and this warp's rows of the state product's left operand are in registers the two key tiles
+  // are dead, and the second stage takes their place (three CTAs fit an SM)
+  auto stage_x = [&](int s) { return s ? aS : bS + 64 * LDK; };
   auto stage_h = [&](int s) { return stage_x(s) + 64 * LDV; };
-  T* yS = stage_x(L::kStages);
+  T* yS = stage_x(0) + L::kStageElems;
   auto stage_g = [&](int s) { return reinterpret_cast<float*>(yS + L::kOutElems) + s * 64; };
-  unsigned char* runs = reinterpret_cast<unsigned char*>(stage_g(L::kStages));
+  unsigned char* runs = reinterpret_cast<unsigned char*>(stage_g(2));
 
   auto issue_head = [&](int hi, int s) {
     const int h = hg * NH + hi;
@@ -314,30 +324,35 @@ __global__ void __launch_bounds__(NT) token_kernel(TokenParams p) {
   issue_head(0, 0);
 
   float scores[8][4];
+  uint32_t rows_a[K / 16][4];  // this warp's 16 rows of a, as A fragments
+  cp_async_wait<0>();
+  __syncthreads();
+#pragma unroll
+  for (int ks = 0; ks < K / 16; ++ks) load_a<T, A_ROW>(rows_a[ks], aS + r0 * LDK, LDK, ks * 16, lane);
+  zero_acc(scores);
+  warp_gemm_ra<T, 8, K / 16, B_NK>(scores, rows_a, bS, LDK, lane);
+  if (NH > 1) __syncthreads();  // the key tiles are free
 #pragma unroll 1
   for (int hi = 0; hi < NH; ++hi) {
-    const int h = hg * NH + hi, s = hi % L::kStages;
+    const int h = hg * NH + hi, s = hi & 1;
     if (NH > 1 && hi + 1 < NH) {
       issue_head(hi + 1, s ^ 1);
-      cp_async_wait<1>();
-    } else {
+      if (hi > 0) cp_async_wait<1>();
+    } else if (NH > 1) {
       cp_async_wait<0>();
     }
-    __syncthreads();
-    if (hi == 0) {
-      zero_acc(scores);
-      warp_gemm<T, 8, K / 16, A_ROW, B_NK>(scores, aS + r0 * LDK, LDK, bS, LDK, lane);
-    }
+    if (NH > 1) __syncthreads();
     const float* Gs = stage_g(s);
     const RowScalars rs0 = row_scalars(Gs, runs, m.flags, r0 + g);
     const RowScalars rs1 = row_scalars(Gs, runs, m.flags, r0 + g + 8);
     float acc[NTV][4];
     zero_acc(acc);
     if (MODE != kZ) {
-      warp_gemm<T, NTV, K / 16, A_ROW, B_KN>(acc, aS + r0 * LDK, LDK, stage_h(s), LDV, lane);
-      const float w0 = MODE == kOut ? rs0.gam : rs0.gamr, w1 = MODE == kOut ? rs1.gam : rs1.gamr;
+      warp_gemm_ra<T, NTV, K / 16, B_KN>(acc, rows_a, stage_h(s), LDV, lane);
 #pragma unroll
-      for (int nt = 0; nt < NTV; ++nt) acc[nt][0] *= w0, acc[nt][1] *= w0, acc[nt][2] *= w1, acc[nt][3] *= w1;
+      for (int nt = 0; nt < NTV; ++nt) {
+        acc[nt][0] *= rs0.gam, acc[nt][1] *= rs0.gam, acc[nt][2] *= rs1.gam, acc[nt][3] *= rs1.gam;
+      }
     }
 #pragma unroll
     for (int ks = 0; ks < 4; ++ks) {  // 16 columns of the score tile at a time, from the diagonal on
@@ -367,8 +382,7 @@ __global__ void __launch_bounds__(NT) token_kernel(TokenParams p) {
         *reinterpret_cast<float2*>(z + 8 * V + nt * 8) = make_float2(acc[nt][2], acc[nt][3]);
       }
     } else {  // through this warp's rows of the staging tile, in 16-byte stores
-      const float w = MODE == kOut ? p.scale : 1.f;
-      store_acc<T, NTV>(yS, LDV, r0, 0, acc, lane, w, w);
+      store_acc<T, NTV>(yS, LDV, r0, 0, acc, lane, p.scale, p.scale);
       __syncwarp();
       const int rows = min(16, m.len - r0);
       if (rows > 0) {
@@ -393,10 +407,10 @@ int run_state(const StateParams& sp, int chains, cudaStream_t s) {
 }
 
 // Value columns per CTA: blocks of 32 shorten a chunk's products and double the CTAs, at the price of reading q, k and Ag
-// once per block; taken while the SMs are not full without it (four CTAs of an SM hide each other's barriers).
+// once per block; taken while blocks of 64 leave most SMs with less than three CTAs to hide each other's barriers.
 template <typename T, int K, bool DELTA, bool BWD>
 int run_state(const StateParams& sp, int chains, cudaStream_t s) {
-  return (long)chains * (sp.V / 64) < 4 * 148 ? run_state<T, K, 32, DELTA, BWD>(sp, chains, s)
+  return (long)chains * (sp.V / 64) <= 2 * 148 ? run_state<T, K, 32, DELTA, BWD>(sp, chains, s)
                                               : run_state<T, K, 64, DELTA, BWD>(sp, chains, s);
 }
 
@@ -423,7 +437,6 @@ int run_tokens(const TokenParams& tp, int nc, cudaStream_t s) {
 template <typename T, int K, int V>
 int run_tokens(const TokenParams& tp, int mode, int nc, cudaStream_t s) {
   if (mode == kOut) return run_tokens<T, K, V, kOut>(tp, nc, s);
-  if (mode == kGrad) return run_tokens<T, K, V, kGrad>(tp, nc, s);
   return run_tokens<T, K, V, kZ>(tp, nc, s);
 }
 
@@ -493,9 +506,9 @@ int launch_split_bwd_state(const ChunkedCtx& c, const jla_bwd_io& io, char* scra
   const Plan& pl = c.plan;
   if (pl.rows == 0) return JLA_OK;
   const bool bf = p.dtype == JLA_DTYPE_BF16;
-  TokenParams tp = token_params(c, pl.delta ? kZ : kGrad);
-  tp.x = io.d_o;
   if (pl.delta) {
+    TokenParams tp = token_params(c, kZ);
+    tp.x = io.d_o;
     tp.y = scratch + pl.z;
     const int rc = bf ? run_tokens<__nv_bfloat16>(tp, p, kZ, pl.nc, s) : run_tokens<__half>(tp, p, kZ, pl.nc, s);
     if (rc != JLA_OK) return rc;
@@ -506,12 +519,8 @@ int launch_split_bwd_state(const ChunkedCtx& c, const jla_bwd_io& io, char* scra
   sp.first = io.d_final, sp.last = io.dh0;
   sp.h = scratch + pl.dh, sp.vn = scratch + pl.dvn, sp.dv = io.dv;
   const int chains = pl.rows * p.H;
-  const int rc = bf ? run_states<__nv_bfloat16, true>(sp, p, pl.delta, chains, s)
-                    : run_states<__half, true>(sp, p, pl.delta, chains, s);
-  if (rc != JLA_OK || pl.delta) return rc;
-  tp.h = scratch + pl.dh;
-  tp.y = io.dv;
-  return bf ? run_tokens<__nv_bfloat16>(tp, p, kGrad, pl.nc, s) : run_tokens<__half>(tp, p, kGrad, pl.nc, s);
+  return bf ? run_states<__nv_bfloat16, true>(sp, p, pl.delta, chains, s)
+            : run_states<__half, true>(sp, p, pl.delta, chains, s);
 }
 
 }  // namespace jla

@@ -191,19 +191,27 @@ template <int N> __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
 }
 
+// 16 bytes, or zeros where `valid` is false (the source is not read then).
+__device__ __forceinline__ void cp_async16_or_zero(void* smem, const void* gmem, bool valid) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_u32(smem)), "l"(gmem), "r"(valid ? 16 : 0));
+}
+
 // Copy a [rows_valid x COLS] 16-bit tile (global row stride `gstride` elements) into smem rows of stride `ld`;
-// rows rows_valid..ROWS-1 are zero-filled. All `nthreads` threads of the CTA call it.
+// rows rows_valid..ROWS-1 are zero-filled. All `nthreads` threads of the CTA call it (a multiple of COLS / 8). A thread
+// keeps its column and steps down the rows, so a copy costs an add, a compare and the copy itself; the missing rows are
+// zero-filled by the copy, without a branch.
 template <typename T, int ROWS, int COLS>
 __device__ __forceinline__ void load_tile_async(T* dst, int ld, const T* src, long gstride, int rows_valid, int tid,
                                                 int nthreads) {
   constexpr int VPR = COLS / 8;  // 16-byte vectors per row
-  for (int idx = tid; idx < ROWS * VPR; idx += nthreads) {
-    const int r = idx / VPR, c = (idx - r * VPR) * 8;
-    if (r < rows_valid) {
-      cp_async16(dst + r * ld + c, src + r * gstride + c);
-    } else {
-      *reinterpret_cast<uint4*>(dst + r * ld + c) = make_uint4(0, 0, 0, 0);
-    }
+  const int c = (tid % VPR) * 8, step = nthreads / VPR;
+  int r = tid / VPR;
+  const T* from = src + r * gstride + c;
+  T* to = dst + r * ld + c;
+#pragma unroll
+  for (int i = 0; i < (ROWS + step - 1) / step; ++i) {
+    if (ROWS % step == 0 || r < ROWS) cp_async16_or_zero(to, from, r < rows_valid);
+    r += step, from += step * gstride, to += step * ld;
   }
 }
 
