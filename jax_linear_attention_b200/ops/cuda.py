@@ -239,10 +239,12 @@ def _forward(q, k, v, g, beta, h0, k_read, cfg: dict, needs_grad: bool):
     res_bytes = lib.jla_residual_bytes(C.byref(p)) if needs_grad else 0
     share = _PassOptions.share if T > 1 else None  # (a single token has no tables to share)
     if share is not None:  # one residual-layout buffer for a run of calls; the first one fills its tables
-        # identity and version of the tensors the CALLER passed (not of the float32 / int32 / contiguous copies
-        # made on the way here, whose addresses can be reused by the allocator inside one shared_prep block)
+        # memory, layout and version of the tensors the CALLER passed (not of the float32 / int32 / contiguous copies made on
+        # the way here). They are kept until the block ends, so their addresses stay theirs; a detached alias, which is how
+        # the differentiated pass of a split gets its leaves, is the same memory at the same version.
         owners = cfg["prep_owners"]
-        identity = tuple((id(x), getattr(x, "_version", 0)) for x in owners)
+        identity = tuple((x.data_ptr(), x._version, x.shape, x.stride(), x.dtype) if isinstance(x, torch.Tensor) else id(x)
+                         for x in owners)
         key = (identity, tuple(q.shape), tuple(v.shape[2:3]), q.dtype, cfg["kind"], cfg["l2norm"],
                cfg["precision"])
         p.flags = flags | _lib.FLAG_SAVE_RESIDUALS
@@ -254,7 +256,7 @@ def _forward(q, k, v, g, beta, h0, k_read, cfg: dict, needs_grad: bool):
             flags |= _lib.FLAG_PREP_DONE
         else:
             share["key"], share["buffer"] = key, torch.empty(full, dtype=torch.uint8, device=dev)
-            share["keep"] = owners  # the keyed objects stay alive, so their ids stay theirs
+            share["keep"] = owners  # the keyed memory stays allocated, so its addresses stay its own
         p.flags = flags
         residuals = share["buffer"] if as_residuals else None
         scratch = None if as_residuals else share["buffer"]
