@@ -424,8 +424,8 @@ __global__ void __launch_bounds__(256, 1) sg_chunk_grads_kernel(BwdParams p) {
 //
 // Sixteen warps in two groups of eight: the query group forms P, dP and the dq terms, the key group the dk terms, <S, dS+>
 // and dV (for which it takes P from the query group). Bound by the latency of its dependent instructions at four warps a
-// scheduler (0.3 issued a cycle, tensor pipe 15 %). Measured at B8 T2048 H64 P64 N128: 674 us; with <S, dS+> in the query
-// group 768 us; as one group of eight warps, two CTAs an SM, both accumulators in every warp (spilling) 709 us; the form
+// scheduler (0.3 issued a cycle, tensor pipe 15 %). Measured at B8 T2048 H64 P64 N128: 588 us; with the score table read from
+// L2 for every head and the document test in every element 674 us; with <S, dS+> in the query group as well 768 us; as one group of eight warps, two CTAs an SM, both accumulators in every warp (spilling) 709 us; the form
 // with a product with K and one with Q per head, and dV in a kernel of its own, 613 + 149 us. The tiles of the next head
 // are on their way for the whole time of one head: one block-wide barrier a head, and a hand-over of P between the groups.
 template <typename T, int K, int V>
@@ -435,7 +435,8 @@ struct DecayGradSmem {
   static constexpr int kStageBytes = kStageElems * 2 + 256;  // + G[64]
   // per-head dG terms: rows [2][64] query group, [2][64] key group, columns [4][64], sums [16], two heads' worth
   static constexpr int kVecFloats = 128 + 128 + 256 + 16;
-  static constexpr int kBytes = (2 * 64 * LDK + 2 * 64 * LDC) * 2 + 2 * kStageBytes + 2 * kVecFloats * 4 + 64;
+  static constexpr int kTabBytes = 64 * 64 * 4;  // the raw scores, in fragment order (walks over heads)
+  static constexpr int kBytes = (2 * 64 * LDK + 2 * 64 * LDC) * 2 + 2 * kStageBytes + 2 * kVecFloats * 4 + 64 + kTabBytes;
   // (K = V = 128, which only an A/B switch sends here, has room for one head's tiles at a time)
   static constexpr bool kTwoStages = kBytes <= 227 * 1024;
   static constexpr int kAllocBytes = kTwoStages ? kBytes : kBytes - kStageBytes;
@@ -465,7 +466,8 @@ __global__ void __launch_bounds__(512, 1) decay_grads_kernel(BwdParams p) {
   unsigned char* vec_base = reinterpret_cast<unsigned char*>(P0 + 2 * 64 * LDC);
   auto vecs = [&](int s) { return reinterpret_cast<float*>(vec_base) + s * L::kVecFloats; };
   unsigned char* runs = vec_base + 2 * L::kVecFloats * 4;
-  unsigned char* stage_base = runs + 64;
+  float* tab = reinterpret_cast<float*>(runs + 64);
+  unsigned char* stage_base = runs + 64 + L::kTabBytes;
   auto stage_s = [&](int s) { return reinterpret_cast<T*>(stage_base + s * L::kStageBytes); };
   auto stage_ds = [&](int s) { return stage_s(s) + K * LDV; };
   auto stage_v = [&](int s) { return stage_ds(s) + K * LDV; };
@@ -476,6 +478,10 @@ __global__ void __launch_bounds__(512, 1) decay_grads_kernel(BwdParams p) {
   load_tile_async<T, 64, K>(qS, LDK, static_cast<const T*>(p.q) + key, (long)p.Hk * K, m.len, tid, NT);
   load_tile_async<T, 64, K>(kS, LDK, static_cast<const T*>(p.k) + key, (long)p.Hk * K, m.len, tid, NT);
   if (tid < 4) cp_async16(runs + tid * 16, p.runs + (long)c * 64 + tid * 16);
+  if (NH > 1) {
+    const float* src = p.qk_tab + ((long)c * p.Hk + hk) * kQkTabFloats;
+    for (int i = tid * 4; i < 64 * 64; i += NT * 4) cp_async16(tab + i, src + i);
+  }
   auto load_head = [&](int hi) {
     const int h = hg * NH + hi, s = hi & 1;
     const long slot = (long)c * p.H + h, val = ((long)m.tok0 * p.H + h) * V;
@@ -524,6 +530,7 @@ __global__ void __launch_bounds__(512, 1) decay_grads_kernel(BwdParams p) {
     if (hi + 1 < NH) load_head(hi + 1);
     if (hi > 0 && p.dg && tid < 32) write_dg(hi - 1);
     const float* Gs = stage_g(s);
+    const bool one_run = runs[63] == 0;  // one document in the chunk
     const RowScalars rs0 = row_scalars(Gs, runs, m.flags, r0 + g);
     const RowScalars rs1 = row_scalars(Gs, runs, m.flags, r0 + g + 8);
     float row0 = 0.f, row1 = 0.f;  // this warp's share of dG for its rows r0 + g and r0 + g + 8
@@ -533,12 +540,11 @@ __global__ void __launch_bounds__(512, 1) decay_grads_kernel(BwdParams p) {
         zero_acc(accP);
         zero_acc(tile);
         if (NH > 1) {
-          const float4* src = reinterpret_cast<const float4*>(p.qk_tab + ((long)c * p.Hk + hk) * kQkTabFloats) +
-                              (quad * 8 + 4 * ch) * 32 + lane;
+          const float4* src = reinterpret_cast<const float4*>(tab) + (quad * 8 + 4 * ch) * 32 + lane;
 #pragma unroll
           for (int nt = 0; nt < 4; ++nt) {
             if (!lower) break;
-            const float4 x = __ldg(src + nt * 32);
+            const float4 x = src[nt * 32];
             tile[nt][0] = x.x, tile[nt][1] = x.y, tile[nt][2] = x.z, tile[nt][3] = x.w;
           }
         } else if (lower) {
@@ -551,7 +557,8 @@ __global__ void __launch_bounds__(512, 1) decay_grads_kernel(BwdParams p) {
           for (int e = 0; e < 4; ++e) {
             const int i = r0 + g + ((e >> 1) << 3), j = cc0 + nt * 8 + 2 * t + (e & 1);
             const RowScalars& rs = (e >> 1) ? rs1 : rs0;
-            const float w = lower ? p.scale * decay_ij(Gs, runs, i, j, rs.G, rs.run) : 0.f;
+            const bool seen = lower && j <= i && (one_run || runs[j] == rs.run);
+            const float w = seen ? p.scale * __expf(rs.G - Gs[j]) : 0.f;
             const float dp = accP[nt][e] * w;
             sumP[nt][e] += dp;
             accP[nt][e] = dp * tile[nt][e];
