@@ -169,7 +169,7 @@ int launch_sg_fwd(const ChunkedCtx& c, const jla_fwd_io& io, cudaStream_t s);
 int launch_split_fwd(const ChunkedCtx& c, const jla_fwd_io& io, cudaStream_t s);        // chunked_split.cu
 int launch_split_bwd_state(const ChunkedCtx& c, const jla_bwd_io& io, char* scratch, cudaStream_t s);
 int launch_sg_bwd(const ChunkedCtx& c, const jla_bwd_io& io, char* scratch, cudaStream_t s);
-int l2norm_fwd(const void* x, void* y, int dtype, long rows, int K, cudaStream_t stream);
+int l2norm_fwd(const void* q, void* qn, const void* k, void* kn, int dtype, long rows, int K, cudaStream_t stream);  // both at once
 int launch_sg_fwd_tc(const ChunkedCtx& c, const jla_fwd_io& io, cudaStream_t s);
 int launch_sg_bwd_state_tc(const ChunkedCtx& c, const jla_bwd_io& io, char* scratch, cudaStream_t s);
 int launch_chunk_grads_tc(const ChunkedCtx& c, const jla_bwd_io& io, char* scratch, bool direct, cudaStream_t s);

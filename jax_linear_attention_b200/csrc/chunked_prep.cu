@@ -312,9 +312,7 @@ int launch_prep(const ChunkedCtx& c, cudaStream_t s) {
   JLA_LAUNCH_OK();
   if (pl.l2norm) {
     const long nrows = (long)p.B * p.T * p.Hk;
-    int rc = l2norm_fwd(p.q, c.res + pl.qn, p.dtype, nrows, p.K, s);
-    if (rc != JLA_OK) return rc;
-    rc = l2norm_fwd(p.k, c.res + pl.kn, p.dtype, nrows, p.K, s);
+    const int rc = l2norm_fwd(p.q, c.res + pl.qn, p.k, c.res + pl.kn, p.dtype, nrows, p.K, s);
     if (rc != JLA_OK) return rc;
   }
   if (shares_scores(p)) {  // grouped simple GLA on the mma.sync kernels: the in-chunk scores once per key head

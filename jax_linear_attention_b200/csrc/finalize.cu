@@ -91,11 +91,22 @@ __global__ void finalize_key_grad_kernel(const float* __restrict__ acc, const T*
   }
 }
 
+// The two tensors of a norm launch (gridDim.y selects): the calls that pass here are often small enough for the launches
+// to count (5003 x 8 x 128: 10.7 us in two launches, 9.2 us in one). dq and dk of the epilogue above stay two launches: in
+// one they took 0.21 instead of 0.17 ms where their accumulators are larger than L2.
+template <typename T>
+struct RowsPair {
+  const T* x[2];
+  T* y[2];
+};
+
 // y = x * rsqrt(sum x^2 + 1e-6), fp32 math, rounded to the tensor dtype (reference.py:65-69). HBM-bound: a row of K
 // channels belongs to K / VEC adjacent lanes with one 16-byte load each, and every lane group has ROWS rows' loads in
 // flight before the first sum (a warp per row with 2-byte loads took 7.8 us for the 10 MB of 5003 x 8 x 128).
 template <typename T, int ROWS>
-__global__ void __launch_bounds__(256) l2norm_fwd_kernel(const T* __restrict__ x, T* __restrict__ y, long rows, int K) {
+__global__ void __launch_bounds__(256) l2norm_fwd_kernel(RowsPair<T> pair, long rows, int K) {
+  const T* __restrict__ x = pair.x[blockIdx.y];
+  T* __restrict__ y = pair.y[blockIdx.y];
   constexpr int VEC = 16 / (int)sizeof(T);
   const int lanes = K / VEC;  // a power of two <= 32 (checked by the launcher)
   const int groups = 256 / lanes;
@@ -129,7 +140,9 @@ __global__ void __launch_bounds__(256) l2norm_fwd_kernel(const T* __restrict__ x
 
 // The same for rows that are not whole groups of 16 aligned bytes: one warp per row, an element at a time.
 template <typename T>
-__global__ void __launch_bounds__(256) l2norm_rows_kernel(const T* __restrict__ x, T* __restrict__ y, long rows, int K) {
+__global__ void __launch_bounds__(256) l2norm_rows_kernel(RowsPair<T> pair, long rows, int K) {
+  const T* __restrict__ x = pair.x[blockIdx.y];
+  T* __restrict__ y = pair.y[blockIdx.y];
   const long row = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   if (row >= rows) return;
   const int lane = threadIdx.x & 31;
@@ -165,21 +178,22 @@ int finalize_t(const float* acc, const void* raw, void* out, long rows, int H, i
   return JLA_OK;
 }
 
+bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
+
 template <typename T>
-int l2norm_t(const void* x, void* y, long rows, int K, cudaStream_t stream) {
+int l2norm_t(const void* q, void* qn, const void* k, void* kn, long rows, int K, cudaStream_t stream) {
   if (rows == 0) return JLA_OK;
   constexpr int kRows = 4;
   const int lanes = K * (int)sizeof(T) / 16;
-  const bool vec = K * sizeof(T) % 16 == 0 && lanes <= 32 && (lanes & (lanes - 1)) == 0 &&
-                   ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0;
+  const bool vec = K * sizeof(T) % 16 == 0 && lanes <= 32 && (lanes & (lanes - 1)) == 0 && aligned16(q) && aligned16(qn) &&
+                   aligned16(k) && aligned16(kn);
+  const RowsPair<T> pair = {{static_cast<const T*>(q), static_cast<const T*>(k)}, {static_cast<T*>(qn), static_cast<T*>(kn)}};
   ProfScope ps(kProfL2Norm, stream);
   if (vec) {
     const long per = 256 / lanes * kRows;
-    l2norm_fwd_kernel<T, kRows><<<(unsigned)((rows + per - 1) / per), 256, 0, stream>>>(static_cast<const T*>(x),
-                                                                                        static_cast<T*>(y), rows, K);
+    l2norm_fwd_kernel<T, kRows><<<dim3((unsigned)((rows + per - 1) / per), 2), 256, 0, stream>>>(pair, rows, K);
   } else {
-    l2norm_rows_kernel<T><<<(unsigned)((rows + 7) / 8), 256, 0, stream>>>(static_cast<const T*>(x), static_cast<T*>(y),
-                                                                         rows, K);
+    l2norm_rows_kernel<T><<<dim3((unsigned)((rows + 7) / 8), 2), 256, 0, stream>>>(pair, rows, K);
   }
   JLA_LAUNCH_OK();
   return JLA_OK;
@@ -199,11 +213,11 @@ int finalize_key_grad(const float* acc, const void* raw, void* out, int dtype, l
   return JLA_ERR_BAD_ARGUMENT;
 }
 
-int l2norm_fwd(const void* x, void* y, int dtype, long rows, int K, cudaStream_t stream) {
+int l2norm_fwd(const void* q, void* qn, const void* k, void* kn, int dtype, long rows, int K, cudaStream_t stream) {
   switch (dtype) {
-    case JLA_DTYPE_BF16: return l2norm_t<__nv_bfloat16>(x, y, rows, K, stream);
-    case JLA_DTYPE_F16: return l2norm_t<__half>(x, y, rows, K, stream);
-    case JLA_DTYPE_F32: return l2norm_t<float>(x, y, rows, K, stream);
+    case JLA_DTYPE_BF16: return l2norm_t<__nv_bfloat16>(q, qn, k, kn, rows, K, stream);
+    case JLA_DTYPE_F16: return l2norm_t<__half>(q, qn, k, kn, rows, K, stream);
+    case JLA_DTYPE_F32: return l2norm_t<float>(q, qn, k, kn, rows, K, stream);
   }
   set_error("unknown dtype %d", dtype);
   return JLA_ERR_BAD_ARGUMENT;
