@@ -208,16 +208,15 @@ __global__ void __launch_bounds__(512, 1) kda_intra_grads_kernel(KdaGradParams p
 #pragma unroll
     for (int ii = 0; ii < 16; ++ii) {
       acc += gv[ii];
-      Gm[(16 * hh + ii) * KD + ch] = acc;
+      gv[ii] = acc;  // (kept in registers until the tokens before are known)
     }
     part[hh * KD + ch] = acc;
     cp_async_wait<0>();
     __syncthreads();
     float off = 0.f;
     for (int b = 0; b < hh; ++b) off += part[b * KD + ch];
-    if (hh > 0) {
-      for (int i = 16 * hh; i < 16 * hh + 16; ++i) Gm[i * KD + ch] += off;
-    }
+#pragma unroll
+    for (int ii = 0; ii < 16; ++ii) Gm[(16 * hh + ii) * KD + ch] = gv[ii] + off;
     const float total = acc + off;
     if (hh == 3) Glast[ch] = total;
     unbounded = __syncthreads_or(hh == 3 && !(fabsf(total) <= kda_bounded_log<T>()));

@@ -92,27 +92,22 @@ __global__ void __launch_bounds__(256, 2) kda_prep_kernel(KdaPrepParams p) {
     const float* gp = p.g + ((long)m.tok0 * p.H + h) * KD + ch;
     const long gstride = (long)p.H * KD;
     float acc = 0.f;
+    float gv[32];  // all loads in flight before the first add; the sums stay here until the other half's total is known
 #pragma unroll
-    for (int i0 = 32 * hh; i0 < 32 * hh + 32; i0 += 16) {
-      float gv[16];  // sixteen loads in flight before the first add
+    for (int ii = 0; ii < 32; ++ii) gv[ii] = (32 * hh + ii < m.len) ? gp[(32 * hh + ii) * gstride] : 0.f;
 #pragma unroll
-      for (int ii = 0; ii < 16; ++ii) gv[ii] = (i0 + ii < m.len) ? gp[(i0 + ii) * gstride] : 0.f;
-#pragma unroll
-      for (int ii = 0; ii < 16; ++ii) {
-        acc += gv[ii];
-        Gm[(i0 + ii) * KD + ch] = acc;
-      }
+    for (int ii = 0; ii < 32; ++ii) {
+      acc += gv[ii];
+      gv[ii] = acc;
     }
     if (hh == 0) M[ch] = acc;  // scratch of the inverse, free until then
     cp_async_wait<0>();
     __syncthreads();
-    float total = acc;
-    if (hh == 1) {
-      const float off = M[ch];
-      for (int i = 32; i < 64; ++i) Gm[i * KD + ch] += off;
-      total = acc + off;
-      Glast[ch] = total;
-    }
+    const float off = hh == 1 ? M[ch] : 0.f;
+#pragma unroll
+    for (int ii = 0; ii < 32; ++ii) Gm[(32 * hh + ii) * KD + ch] = gv[ii] + off;
+    const float total = acc + off;
+    if (hh == 1) Glast[ch] = total;
     unbounded = __syncthreads_or(hh == 1 && !(fabsf(total) <= kda_bounded_log<T>()));
   }
   const bool entering = !(m.flags & 1);
