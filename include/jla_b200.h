@@ -244,6 +244,11 @@ int jla_short_conv_bwd(int dtype, int B, int T, int C, int K, int head_dim, int 
                        const float* weight, const float* bias, const int32_t* segment_ids, const void* state,
                        const void* dy, void* dx, float* dweight, float* dbias, void* dstate, jla_stream_t stream);
 
+/* The state that the next call takes: the last K - 1 rows of x_ext (jla_short_conv_fwd), zero where a row belongs to an
+ * earlier document than the last token. T >= 1, K >= 2; state may be NULL (zeros). src/jla/layers/conv.py:190-210. */
+int jla_short_conv_state(int dtype, int B, int T, int C, int K, const void* x, const int32_t* segment_ids,
+                         const void* state, void* new_state, jla_stream_t stream);
+
 /* Gated RMS norm behind the kernels (the mixers' output norm; with norm_before_gate = 0 the Mamba-2 norm), forward
  * and backward in one pass each; replaces GatedRMSNorm.__call__ (src/jla/layers/norm.py:60-112) and its transpose.
  *   gate = silu(z), or sigmoid(z) with sigmoid_gate;  u = x (norm_before_gate) or x * gate;

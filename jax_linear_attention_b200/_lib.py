@@ -89,6 +89,7 @@ def load() -> C.CDLL:
     int_, i64, ptr, f32 = C.c_int, C.c_int64, C.c_void_p, C.c_float
     for name, types in {  # typed, so that callers pass plain integers (data pointers) and None
         "jla_short_conv_fwd": [int_] * 7 + [ptr] * 7, "jla_short_conv_bwd": [int_] * 7 + [ptr] * 11,
+        "jla_short_conv_state": [int_] * 5 + [ptr] * 5,
         "jla_gate_prologue_fwd": [int_, i64, int_, int_] + [ptr] * 4 + [int_] + [ptr] * 3,
         "jla_gate_prologue_bwd": [int_, i64, int_, int_] + [ptr] * 4 + [int_] + [ptr] * 7,
         "jla_gated_rmsnorm_fwd": [int_, i64, int_, int_] + [ptr] * 3 + [f32, int_, int_] + [ptr] * 2,

@@ -49,6 +49,34 @@ __device__ __forceinline__ float fast_rsqrt(float x) {
   return y;
 }
 
+// Two channels in one 64-bit register pair: sm_100's packed fp32 instructions, each half rounded like the scalar one.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2f(float lo, float hi) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2f(f32x2 x) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(x));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
 // Asynchronous copy of one thread's row (BYTES = 8, 16 or 32) from global to shared memory; `valid` false writes
 // zeros without reading. One commit per group of rows, cp_async_wait_groups<N> leaves the N newest groups in flight.
 template <int BYTES>

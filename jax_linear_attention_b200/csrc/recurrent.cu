@@ -180,35 +180,7 @@ struct Stage {
   }
 };
 
-// Two channels in one 64-bit register pair: sm_100's packed fp32 instructions, each half rounded like the scalar one.
-// The walks issue half the arithmetic instructions this way, which is what is left of a token next to its chain.
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pack2f(float lo, float hi) {
-  f32x2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-  return r;
-}
-__device__ __forceinline__ float2 unpack2f(f32x2 x) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(x));
-  return r;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-  f32x2 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
-  f32x2 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
-  f32x2 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-
+// (packed: the walks issue half the arithmetic instructions, which is what is left of a token next to its chain)
 constexpr int KP2 = KPT / 2;
 typedef f32x2 Chan[KP2];  // the channels of a thread
 

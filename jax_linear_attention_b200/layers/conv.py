@@ -96,5 +96,10 @@ def short_conv(x, weight, bias=None, *, activation: bool = True, head_dim: int |
     y = _ShortConv.apply(x.contiguous(), weight.float().contiguous(), None if bias is None else bias.float().contiguous(),
                          st, seg, int(head_dim or 0), bool(activation))
     with torch.no_grad():
-        new_state = _final_state(x, state, segment_ids, K)
+        if segment_ids is not None and T > 0 and K > 1 and (state is None or state.dtype == x.dtype):
+            x, state = x.detach().contiguous(), None if state is None else state.detach().contiguous()
+            new_state = torch.empty(B, K - 1, Cn, dtype=x.dtype, device=x.device)
+            _call("jla_short_conv_state", x, _DTYPES[x.dtype], B, T, Cn, K, _ptr(x), _ptr(seg), _ptr(state), _ptr(new_state))
+        else:
+            new_state = _final_state(x, state, segment_ids, K)
     return y, new_state
