@@ -147,6 +147,8 @@ _MAX_ANSWERS = 1024
 def _reason(kind: str, q, k, v, gates: tuple, options: dict):
     """``unsupported_reason`` through a table of the signatures already answered: the answer depends on nothing but the
     shapes, dtypes and option values in the key. (A decoding loop asks the same question for every token and layer.)"""
+    if not all(x is None or isinstance(x, (torch.Tensor, str, int, float)) for x in options.values()):
+        return unsupported_reason(kind, q, k, v, gates, options)  # (nothing else goes into a key)
     try:
         key = (kind, q.shape, q.dtype, k.shape, k.dtype, v.shape, v.dtype, *(g.shape for g in gates),
                *((n, x.shape, x.dtype) if isinstance(x, torch.Tensor) else (n, x) for n, x in options.items()
