@@ -528,7 +528,7 @@ __global__ void __launch_bounds__(512, 1) decay_grads_kernel(BwdParams p) {
     cp_async_wait<0>();
     __syncthreads();  // the head's tiles have landed; the head before is done with its own
     if (hi + 1 < NH) load_head(hi + 1);
-    if (hi > 0 && p.dg && tid < 32) write_dg(hi - 1);
+    if (hi > 0 && p.dg && keys && warp == 0) write_dg(hi - 1);  // (the key group has the shorter way)
     const float* Gs = stage_g(s);
     const bool one_run = runs[63] == 0;  // one document in the chunk
     const RowScalars rs0 = row_scalars(Gs, runs, m.flags, r0 + g);
@@ -648,12 +648,8 @@ __global__ void __launch_bounds__(512, 1) decay_grads_kernel(BwdParams p) {
       if (lane == 0) out[512 + warp] = keep_gamma(Gs, runs, m.flags) * part;
       asm volatile("bar.sync 1, 512;" ::: "memory");
       warp_gemm<T, ONT, 4, A_COL, B_KN>(x, Ps + r0, LDC, stage_do(s) + c0, LDV, lane);
-      T* dv = static_cast<T*>(p.dv_out) + ((long)(m.tok0 + r0 + g) * p.H + h) * V + c0 + 2 * t;
-#pragma unroll
-      for (int nt = 0; nt < ONT; ++nt) {
-        if (r0 + g < m.len) *reinterpret_cast<uint32_t*>(dv + nt * 8) = pack2<T>(x[nt][0], x[nt][1]);
-        if (r0 + g + 8 < m.len) *reinterpret_cast<uint32_t*>(dv + (long)8 * p.H * V + nt * 8) = pack2<T>(x[nt][2], x[nt][3]);
-      }
+      store_acc_wide<T, ONT>(static_cast<T*>(p.dv_out) + ((long)(m.tok0 + r0) * p.H + h) * V + c0, (long)p.H * V, x, lane,
+                             m.len - r0);
     }
     if (t == 0) {
       float* rows = out + (keys ? 128 : 0) + ch * 64 + r0 + g;

@@ -188,21 +188,15 @@ __global__ void __launch_bounds__(NT) state_kernel(StateParams p) {
         zero_acc(x);
         warp_gemm<T, NTV, 4, A_COL, B_KN>(x, stage_ag(s) + r0, LDC, A2, LDV, lane);  // dW = dV = Ag^T dVn
         store_acc<T, NTV>(A1, LDV, r0, 0, x, lane, -rs0.gam, -rs1.gam);
-        T* dv = static_cast<T*>(p.dv) + ((long)(m.tok0 + r0 + g) * p.H + h) * p.V + v0 + 2 * t;
-#pragma unroll
-        for (int nt = 0; nt < NTV; ++nt) {
-          if (r0 + g < m.len) *reinterpret_cast<uint32_t*>(dv + nt * 8) = pack2<T>(x[nt][0], x[nt][1]);
-          if (r0 + g + 8 < m.len) {
-            *reinterpret_cast<uint32_t*>(dv + (long)8 * p.H * p.V + nt * 8) = pack2<T>(x[nt][2], x[nt][3]);
-          }
-        }
+        store_acc_wide<T, NTV>(static_cast<T*>(p.dv) + ((long)(m.tok0 + r0) * p.H + h) * p.V + v0, (long)p.H * p.V, x, lane,
+                               m.len - r0);
       }
     } else {
       __syncthreads();
       // straight from the accumulators: a 16-bit copy in shared memory would leave room for one CTA less on an SM
 #pragma unroll
       for (int mt = 0; mt < MT; ++mt) {
-        store_acc<T, NTV>(hout, p.V, sr0 + 16 * mt, 0, acc[mt], lane);
+        store_acc_wide<T, NTV>(hout + (long)(sr0 + 16 * mt) * p.V, p.V, acc[mt], lane, 16);
       }
     }
 #pragma unroll
