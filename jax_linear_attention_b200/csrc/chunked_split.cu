@@ -15,7 +15,7 @@
 // blocks of VB. What is read back for the outputs (h, Vn) the backward keeps anyway. Forwards that keep nothing stay on
 // the fused kernel (chunked_fwd.cu), which needs no scratch for h.
 //
-// Measured: the walks of the d = 64 shape 23 + 33 us (fused 109 + 119), of the Mamba-2 shape 175 + 170 us and its outputs
+// Measured: the walks of the d = 64 shape 23 + 29 us (fused 109 + 119), of the Mamba-2 shape 139 + 137 us and its outputs
 // 150 us (fused 439 + 436); what bounds them now is the latency of a chunk's loads, barriers and products at one to four
 // CTAs of four warps an SM.
 //
