@@ -112,7 +112,12 @@ __global__ void __launch_bounds__(256, 1) kda_state_grads_kernel(KdaGradParams p
     float acc[4][4];
     zero_acc(acc);  // dP = scale dO Vn^T
     warp_gemm<T, 4, VD / 16, A_ROW, B_KN>(acc, dOs + r0 * LDV, LDV, vnS + cc0, LDC, lane);
-    store_acc<T, 4>(static_cast<T*>(p.dp) + slot * 4096, 64, r0, cc0, acc, lane, p.scale, p.scale);
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[nt][e] *= p.scale;
+    }
+    store_acc_wide<T, 4>(static_cast<T*>(p.dp) + slot * 4096 + r0 * 64 + cc0, 64, acc, lane, 16);
   }
   cp_async_wait<0>();
   __syncthreads();
@@ -126,7 +131,7 @@ __global__ void __launch_bounds__(256, 1) kda_state_grads_kernel(KdaGradParams p
     float acc[4][4];
     zero_acc(acc);  // dAg = dVn W^T
     warp_gemm<T, 4, VD / 16, A_COL, B_KN>(acc, dvnS + r0, LDC, wS + cc0, LDC, lane);
-    store_acc<T, 4>(static_cast<T*>(p.dag) + slot * 4096, 64, r0, cc0, acc, lane);
+    store_acc_wide<T, 4>(static_cast<T*>(p.dag) + slot * 4096 + r0 * 64 + cc0, 64, acc, lane, 16);
   }
   {  // dd[c] = sum_v dS+[c][v] S[c][v]
     const int col = tid & (KD - 1), half = tid >> 7;
@@ -328,6 +333,7 @@ __global__ void __launch_bounds__(512, 1) kda_intra_grads_kernel(KdaGradParams p
         sgu[nt & 1][hi] = *reinterpret_cast<const float2*>(dku + off);
       }
     };
+    uint32_t wq[2][4], wk[2][4], wr[2][RK ? 4 : 1];  // dq, dk (and the read key's) of rows i0, i1, packed
     request(0);
     warp_gemm<T, 4, 4, A_ROW, B_KN>(accU, Xm + r0 * LDC, LDC, tb + kc0, LDK, lane);   // dA k~
     warp_gemm<T, 4, 4, A_ROW, B_KN>(accQ, Xp + r0 * LDC, LDC, tb + kc0, LDK, lane);   // dP k~
@@ -374,22 +380,28 @@ __global__ void __launch_bounds__(512, 1) kda_intra_grads_kernel(KdaGradParams p
           dkv[x] = RK ? dkw : dkr + dkw;
           dkrv[x] = dkr;
         }
-        if (i < m.len) {
-          if (dq16) {
-            *reinterpret_cast<uint32_t*>(dq16 + (long)i * kstride + col) = pack2<T>(dqv[0], dqv[1]);
-            *reinterpret_cast<uint32_t*>(dk16 + (long)i * kstride + col) = pack2<T>(dkv[0], dkv[1]);
-          } else {
-            *reinterpret_cast<float2*>(p.dq_acc + tokbase + i * tstride + col) = make_float2(dqv[0], dqv[1]);
-            *reinterpret_cast<float2*>(p.dk_acc + tokbase + i * tstride + col) = make_float2(dkv[0], dkv[1]);
-          }
-          if (RK) *reinterpret_cast<uint32_t*>(dkr16 + (long)i * tstride + col) = pack2<T>(dkrv[0], dkrv[1]);
+        if (!dq16 && i < m.len) {
+          *reinterpret_cast<float2*>(p.dq_acc + tokbase + i * tstride + col) = make_float2(dqv[0], dqv[1]);
+          *reinterpret_cast<float2*>(p.dk_acc + tokbase + i * tstride + col) = make_float2(dkv[0], dkv[1]);
         }
+        wq[hi][nt] = pack2<T>(dqv[0], dqv[1]);
+        wk[hi][nt] = pack2<T>(dkv[0], dkv[1]);
+        if constexpr (RK) wr[hi][nt] = pack2<T>(dkrv[0], dkrv[1]);
       }
       const float a = col_reduce(colsum[0]), b = col_reduce(colsum[1]);
       if (lane < 4) {
         part[rw * KD + kc0 + nt * 8 + 2 * lane] = a;
         part[rw * KD + kc0 + nt * 8 + 2 * lane + 1] = b;
       }
+    }
+#pragma unroll
+    for (int hi = 0; hi < 2; ++hi) {
+      const int i = hi ? i1 : i0;
+      if (dq16) {
+        store_row_words<T>(dq16 + (long)i * kstride + kc0, wq[hi], t, i < m.len);
+        store_row_words<T>(dk16 + (long)i * kstride + kc0, wk[hi], t, i < m.len);
+      }
+      if constexpr (RK) store_row_words<T>(dkr16 + (long)i * tstride + kc0, wr[hi], t, i < m.len);
     }
     db0 += __shfl_xor_sync(0xffffffffu, db0, 1);
     db0 += __shfl_xor_sync(0xffffffffu, db0, 2);
