@@ -176,20 +176,21 @@ def _supports(kind: str):
 class _PassOptions:
     """Process-wide switches for callers that run several passes over the same tokens (the piecewise
     sequence-parallel form). Plain module state, not thread-local: autograd runs backward on its own thread."""
-    share = None              # dict(key=..., buffer=...) while shared_prep() is active
+    share = None              # per value width a dict(key=..., buffer=..., keep=...) while shared_prep() is active
     state_grads_only = False  # backward runs the reverse state pass only (dh0, dv)
     final_state_only = False  # forward computes the final state only (o is left unwritten)
 
 
 class shared_prep:
     """``with shared_prep():`` lets successive forward calls on the same ``k``, gates and document layout (and, with
-    the in-op L2 norm, the same ``q``) share one residual-layout buffer, so that only the first of them computes the
-    chunk table, the gate cumsums and the triangular inverses. Every call overwrites the buffer's state residuals:
-    only the last call inside the block may be differentiated."""
+    the in-op L2 norm, the same ``q``) share one residual-layout buffer per value width, so that only the first of them
+    computes the chunk table, the gate cumsums and the triangular inverses. (The width decides which kernels a call runs,
+    hence which tables there are and where: calls of different widths share nothing.) Every call overwrites the buffer's
+    state residuals: only the last call inside the block may be differentiated."""
 
     def __enter__(self):
         self._outer = _PassOptions.share
-        _PassOptions.share = dict(key=None, buffer=None)
+        _PassOptions.share = {}
         return self
 
     def __exit__(self, *exc):
@@ -241,6 +242,7 @@ def _forward(q, k, v, g, beta, h0, k_read, cfg: dict, needs_grad: bool):
     res_bytes = lib.jla_residual_bytes(C.byref(p)) if needs_grad else 0
     share = _PassOptions.share if T > 1 else None  # (a single token has no tables to share)
     if share is not None:  # one residual-layout buffer for a run of calls; the first one fills its tables
+        share = share.setdefault(V, dict(key=None, buffer=None))
         # memory, layout and version of the tensors the CALLER passed (not of the float32 / int32 / contiguous copies made on
         # the way here). They are kept until the block ends, so their addresses stay theirs; a detached alias, which is how
         # the differentiated pass of a split gets its leaves, is the same memory at the same version.

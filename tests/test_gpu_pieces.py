@@ -106,3 +106,22 @@ def test_documents_shorter_than_a_piece_run_as_plain_rows(monkeypatch):
         assert rel_l2(split[name], plain[name]) < 1e-2, (name, rel_l2(split[name], plain[name]))
     want = run_oracle("gated_deltanet", case, scale=case["meta"]["scale"], chunked=True)
     compare(split, want, 1e-2, "documents as rows")
+
+
+@pytest.mark.parametrize("kind,H,Hk", [("simple_gla", 8, 1), ("gated_deltanet", 4, 2)])
+def test_pieces_of_narrow_values_keep_their_own_tables(kind, H, Hk):
+    """Values of 64 channels next to keys of 128: the map pass of the split runs other kernels, with other tables, than the
+    passes around it. A document over several pieces against the unsplit call (16-bit operands of either: 1e-2)."""
+    from jax_linear_attention_b200.distributed.context_parallel import context_parallel_linear_attention
+
+    case = make_case(kind, B=1, T=1100, H=H, Hk=Hk, K=128, V=64, seed=83, h0=True, gates="baseline")
+    plain = run_cuda(kind, case, scale=case["meta"]["scale"], dtype="bfloat16")
+    t = {n: torch.tensor(case[n], device="cuda", dtype=torch.bfloat16, requires_grad=True) for n in ("q", "k", "v")}
+    t.update({n: torch.tensor(case[n], device="cuda", requires_grad=True) for n in ("g", "beta", "h0") if n in case})
+    gates = {n: t[n] for n in ("g", "beta") if n in t}
+    o, ht = context_parallel_linear_attention(kind, t["q"], t["k"], t["v"], group=False, piece_len=256, impl="cuda",
+                                              scale=case["meta"]["scale"], initial_state=t["h0"], output_final_state=True, **gates)
+    grads = torch.autograd.grad([o, ht], list(t.values()), [torch.tensor(case["do"], device="cuda", dtype=torch.bfloat16),
+                                                            torch.tensor(case["dht"], device="cuda", dtype=torch.float32)])
+    got = {"o": o.detach(), "ht": ht.detach(), **{"d" + n: x for n, x in zip(t, grads)}}
+    compare({n: x.float().cpu().numpy() for n, x in got.items()}, plain, 1e-2, f"{kind} pieces")

@@ -1,0 +1,40 @@
+"""CPU tests of the host's routing rules: what it asks of the library is looked at, nothing is launched."""
+
+import pytest
+import torch
+
+from jax_linear_attention_b200 import _lib
+from jax_linear_attention_b200.ops import cuda
+
+
+@pytest.fixture
+def launches(monkeypatch):
+    """The calls that would have been launched: ``(entry point, arguments)``."""
+    calls = []
+    monkeypatch.setattr(_lib, "launch", lambda name, device, *args: calls.append((name, args)))
+    return calls
+
+
+def _prologues(launches):
+    """Per forward: whether it relies on an earlier prologue, and the buffer that holds the tables."""
+    forwards = [args for name, args in launches if name == "jla_linear_attention_fwd"]
+    return [(bool(p.flags & _lib.FLAG_PREP_DONE), io.residuals or io.scratch) for p, io in forwards]
+
+
+@pytest.mark.parametrize("kind,H,Hk", [("simple_gla", 8, 1), ("gated_deltanet", 2, 2)])
+def test_shared_prologue_belongs_to_a_value_width(launches, kind, H, Hk):
+    """The value width decides which kernels run and which tables the prologue leaves behind (values of 64 next to keys of
+    128 and the 128 x 128 map pass of a split sequence share neither): a pass reuses the tables of its own width only, and
+    finds them again after a pass of another width."""
+    T, K = 128, 128
+    q, k = torch.zeros(1, T, Hk, K, dtype=torch.bfloat16), torch.zeros(1, T, Hk, K, dtype=torch.bfloat16)
+    g, beta = torch.zeros(1, T, H), None if kind == "simple_gla" else torch.zeros(1, T, H)
+    cfg = dict(kind=kind, scale=1.0, l2norm=False, precision=None, output_final_state=True, cu_seqlens=None,
+               segment_ids=None, prep_owners=(k, g, beta, None, None, None))
+    narrow, wide = (torch.zeros(1, T, H, V, dtype=torch.bfloat16) for V in (64, 128))
+    with cuda.shared_prep():
+        for v, needs_grad in ((narrow, False), (wide, False), (narrow, True), (wide, False)):
+            cuda._forward(q, k, v, g, beta, None, None, cfg, needs_grad)
+    (done0, narrow0), (done1, wide1), (done2, narrow2), (done3, wide3) = _prologues(launches)
+    assert [done0, done1, done2, done3] == [False, False, True, True]
+    assert narrow2 == narrow0 and wide3 == wide1 and narrow0 != wide1
