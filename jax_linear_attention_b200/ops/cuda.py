@@ -182,8 +182,8 @@ class _PassOptions:
 
 
 class shared_prep:
-    """``with shared_prep():`` lets successive forward calls on the same ``k``, gates and document layout (and, with
-    the in-op L2 norm, the same ``q``) share one residual-layout buffer per value width, so that only the first of them
+    """``with shared_prep():`` lets successive forward calls on the same ``k``, gates and document layout (and, where the
+    prologue reads it, the same ``q``) share one residual-layout buffer per value width, so that only the first of them
     computes the chunk table, the gate cumsums and the triangular inverses. (The width decides which kernels a call runs,
     hence which tables there are and where: calls of different widths share nothing.) Every call overwrites the buffer's
     state residuals: only the last call inside the block may be differentiated."""
@@ -483,7 +483,9 @@ def _run(kind: str, q, k, v, g, beta, *, scale, initial_state, output_final_stat
                              f"{cu_host.tolist()[:8]}{'...' if cu_host.numel() > 8 else ''}")
     cfg = dict(kind=kind, scale=float(scale), l2norm=bool(use_qk_l2norm), precision=precision,
                output_final_state=bool(output_final_state), cu_seqlens=i32(cu_seqlens), segment_ids=i32(segment_ids),
-               prep_owners=(k, g, beta, segment_ids, cu_seqlens, q if use_qk_l2norm else None))
+               # what the prologue reads: q too where it norms it, folds gates into it (KDA) or forms scores (simple GLA)
+               prep_owners=(k, g, beta, segment_ids, cu_seqlens,
+                            q if use_qk_l2norm or kind in ("kda", "simple_gla") else None))
     inputs = (q.contiguous(), k.contiguous(), v.contiguous(), f32(g), f32(beta), f32(initial_state),
               None if k_read is None else k_read.contiguous())
     if _bypasses_autograd(inputs):  # nothing to differentiate: a decoding step spends a third of its time in apply()

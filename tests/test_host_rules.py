@@ -38,3 +38,20 @@ def test_shared_prologue_belongs_to_a_value_width(launches, kind, H, Hk):
     (done0, narrow0), (done1, wide1), (done2, narrow2), (done3, wide3) = _prologues(launches)
     assert [done0, done1, done2, done3] == [False, False, True, True]
     assert narrow2 == narrow0 and wide3 == wide1 and narrow0 != wide1
+
+
+@pytest.mark.parametrize("kind,V,l2norm", [("kda", 128, False), ("simple_gla", 64, False), ("gated_deltanet", 128, True)])
+def test_shared_prologue_belongs_to_its_queries(launches, monkeypatch, kind, V, l2norm):
+    """Where the prologue works on q too (KDA folds the gates into it, simple GLA's score table, the in-op norm), another q
+    means another prologue."""
+    T, H, K = 128, 4, 128
+    monkeypatch.setattr(torch.Tensor, "is_cuda", property(lambda self: True), raising=False)
+    q, q2, k = (torch.zeros(1, T, 2 if kind == "simple_gla" else H, K, dtype=torch.bfloat16) for _ in range(3))
+    v = torch.zeros(1, T, H, V, dtype=torch.bfloat16)
+    g = torch.zeros(1, T, H, K) if kind == "kda" else torch.zeros(1, T, H)
+    beta = None if kind == "simple_gla" else torch.zeros(1, T, H)
+    with cuda.shared_prep():
+        for x in (q, q, q2):
+            cuda._run(kind, x, k, v, g, beta, scale=1.0, initial_state=None, output_final_state=True, cu_seqlens=None,
+                      segment_ids=None, use_qk_l2norm=l2norm)
+    assert [done for done, _ in _prologues(launches)] == [False, True, False]
