@@ -136,7 +136,8 @@ int jla_abi_version(void);
 const char* jla_last_error(void);
 
 /* NULL if the library has a kernel for `p`, else the reason as text. Of the pointers in `p` only k_read is looked
- * at, and only whether it is NULL (a call with a read key takes another path).
+ * at, and only whether it is NULL (a call with a read key takes another path). Without JLA_FLAG_SAVE_RESIDUALS the
+ * question is about the forward alone (a decoding step, T = 1, runs at head sizes that have no backward).
  * Mirrors unsupported_reason() of src/jla/ops/mosaic_gpu/scalar_gate.py:476-515 and
  * src/jla/ops/mosaic_gpu/vector_gate_ops.py:262-304. */
 const char* jla_unsupported_reason(const jla_problem* p);

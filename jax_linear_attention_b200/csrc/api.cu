@@ -61,13 +61,14 @@ const char* shape_problem(const jla_problem& p) {
   return nullptr;
 }
 
-const char* unsupported(const jla_problem& p) {
+// `forward`: the question is about a forward alone, which for a decoding step is a kernel of its own (with no backward).
+const char* unsupported(const jla_problem& p, bool forward) {
   if (const char* why = shape_problem(p)) return why;
-  if (token_step_applies(p)) return nullptr;
+  if (forward && token_step_applies(p)) return nullptr;
   return resolve_path(p) == JLA_PATH_RECURRENT ? recurrent_unsupported(p) : chunked_unsupported(p);
 }
 
-int check_common(const jla_problem* p) {
+int check_common(const jla_problem* p, bool forward) {
   if (!p) {
     set_error("null problem");
     return JLA_ERR_BAD_ARGUMENT;
@@ -76,7 +77,7 @@ int check_common(const jla_problem* p) {
     set_error("%s", why);
     return JLA_ERR_BAD_ARGUMENT;
   }
-  if (const char* why = unsupported(*p)) {
+  if (const char* why = unsupported(*p, forward)) {
     set_error("%s", why);
     return JLA_ERR_UNSUPPORTED;
   }
@@ -119,26 +120,26 @@ int jla_abi_version(void) { return 1001; }
 
 const char* jla_last_error(void) { return g_error; }
 
-const char* jla_unsupported_reason(const jla_problem* p) { return p ? unsupported(*p) : "null problem"; }
+const char* jla_unsupported_reason(const jla_problem* p) { return p ? unsupported(*p, true) : "null problem"; }
 
 size_t jla_residual_bytes(const jla_problem* p) {
-  if (!p || unsupported(*p) || (p->kind == JLA_KIND_KDA && kda_scan_backward())) return 0;
+  if (!p || unsupported(*p, false) || (p->kind == JLA_KIND_KDA && kda_scan_backward())) return 0;
   return resolve_path(*p) == JLA_PATH_RECURRENT ? 0 : chunked_residual_bytes(*p);
 }
 
 size_t jla_fwd_scratch_bytes(const jla_problem* p) {
-  if (!p || unsupported(*p) || token_step_applies(*p)) return 0;
+  if (!p || unsupported(*p, true) || token_step_applies(*p)) return 0;
   return resolve_path(*p) == JLA_PATH_RECURRENT ? 0 : chunked_fwd_scratch_bytes(*p);
 }
 
 size_t jla_bwd_scratch_bytes(const jla_problem* p) {
-  if (!p || unsupported(*p)) return 0;
+  if (!p || unsupported(*p, false)) return 0;
   return resolve_path(*p, true) == JLA_PATH_RECURRENT ? recurrent_bwd_scratch_bytes(*p) : chunked_bwd_scratch_bytes(*p);
 }
 
 int jla_linear_attention_fwd(const jla_problem* p, const jla_fwd_io* io, jla_stream_t stream) {
   g_error[0] = 0;
-  if (int rc = check_common(p)) return rc;
+  if (int rc = check_common(p, true)) return rc;
   if (!io || ((long)p->B * p->T > 0 && !io->o)) {
     set_error("null output");
     return JLA_ERR_BAD_ARGUMENT;
@@ -150,7 +151,7 @@ int jla_linear_attention_fwd(const jla_problem* p, const jla_fwd_io* io, jla_str
 
 int jla_linear_attention_bwd(const jla_problem* p, const jla_bwd_io* io, jla_stream_t stream) {
   g_error[0] = 0;
-  if (int rc = check_common(p)) return rc;
+  if (int rc = check_common(p, false)) return rc;
   const bool has_tokens = (long)p->B * p->T > 0;
   if (!io || (has_tokens && (!io->d_o || !io->dq || !io->dk || !io->dv))) {
     set_error("null gradient buffer");

@@ -70,6 +70,27 @@ def test_unsupported_reason_and_sizes_without_a_gpu():
     assert rc == _lib.ERR_BAD_ARGUMENT and b"batch size 1" in lib.jla_last_error()
 
 
+@pytest.mark.parametrize("kind,K,V", [("gated_deltanet", 256, 512), ("simple_gla", 128, 192), ("kda", 128, 512)])
+def test_a_decoding_step_has_no_backward(kind, K, V):
+    """Head sizes that only the decoding-step kernel covers: the forward is accepted, nothing of a backward is."""
+    from jax_linear_attention_b200 import _lib
+
+    lib = _lib.load()
+    p = _lib.Problem()
+    p.kind, p.dtype, p.path, p.flags = _lib.KIND[kind], 0, 0, 0
+    p.B, p.T, p.H, p.Hk, p.K, p.V, p.num_seqs, p.scale = 2, 1, 4, 4, K, V, 0, 1.0
+    p.q = p.k = p.v = p.g = p.beta = 16  # (never read: nothing is launched)
+    assert _lib.unsupported_reason(p) is None
+    assert lib.jla_fwd_scratch_bytes(ctypes.byref(p)) == 0
+    assert lib.jla_residual_bytes(ctypes.byref(p)) == 0
+    assert lib.jla_bwd_scratch_bytes(ctypes.byref(p)) == 0
+    io = _lib.BwdIO()
+    io.d_o = io.dq = io.dk = io.dv = io.dg = io.dbeta = 16
+    assert lib.jla_linear_attention_bwd(ctypes.byref(p), ctypes.byref(io), None) == _lib.ERR_UNSUPPORTED
+    p.flags = _lib.FLAG_SAVE_RESIDUALS
+    assert _lib.unsupported_reason(p) is not None
+
+
 def test_dispatcher_mirrors_reference_errors():
     from jax_linear_attention_b200 import ops
 
