@@ -54,9 +54,10 @@ __global__ void __launch_bounds__(NT) token_step_kernel(StepParams p) {
   __shared__ float4 red[2][NG][CT];
   __shared__ float qk_s;
   const int tid = threadIdx.x, lane = tid & 31, cg = tid % CT, ng = tid / CT;
-  const int vblocks = p.V / VB;
-  const int h = blockIdx.x / vblocks, v0 = (blockIdx.x - h * vblocks) * VB + 4 * cg;
-  const long row = (long)blockIdx.y * p.H + h;  // (batch row, value head)
+  const int vblocks = p.V / VB, per_row = p.H * vblocks;
+  const int b = blockIdx.x / per_row, hc = blockIdx.x - b * per_row;  // batch row; its head and block of columns
+  const int h = hc / vblocks, v0 = (hc - h * vblocks) * VB + 4 * cg;
+  const long row = (long)b * p.H + h;  // (batch row, value head)
   const int hk = h / (p.H / p.Hk);
 
   float4 S[RPT];
@@ -75,7 +76,7 @@ __global__ void __launch_bounds__(NT) token_step_kernel(StepParams p) {
   }
 
   if (tid < 32) {
-    const long key = ((long)blockIdx.y * p.Hk + hk) * K;
+    const long key = ((long)b * p.Hk + hk) * K;
     float q[KPL], k[KPL];
     float sq = 0.f, sk = 0.f;
 #pragma unroll
@@ -187,8 +188,7 @@ int launch_gate(const StepParams& sp, int kind, dim3 grid, cudaStream_t s) {
 template <typename T>
 int launch_dims(const StepParams& sp, const jla_problem& p, cudaStream_t s) {
   const int vb = p.V % 128 == 0 ? 128 : 64;
-  // rows go on gridDim.y (at most 65535 of them per launch: token_step_applies)
-  const dim3 grid((unsigned)(p.H * (p.V / vb)), (unsigned)p.B);
+  const dim3 grid((unsigned)((long)p.B * p.H * (p.V / vb)));  // (below 2^31: token_step_applies)
   switch (p.K) {
     case 64: return vb == 128 ? launch_gate<T, 64, 128>(sp, p.kind, grid, s) : launch_gate<T, 64, 64>(sp, p.kind, grid, s);
     case 128: return vb == 128 ? launch_gate<T, 128, 128>(sp, p.kind, grid, s) : launch_gate<T, 128, 64>(sp, p.kind, grid, s);
@@ -223,9 +223,9 @@ int launch_dtype(const StepParams& sp, const jla_problem& p, cudaStream_t s) {
 // row's state, so segment_ids do not matter), nothing to keep for a backward, states in whole 16-byte groups. The
 // explicitly requested chunk kernels (JLA_PATH_CHUNKED) are left alone.
 bool token_step_applies(const jla_problem& p) {
-  return p.T == 1 && p.B > 0 && p.B <= 65535 && p.num_seqs == 0 && p.path != JLA_PATH_CHUNKED &&
+  return p.T == 1 && p.B > 0 && p.num_seqs == 0 && p.path != JLA_PATH_CHUNKED &&
          !(p.flags & (JLA_FLAG_SAVE_RESIDUALS | JLA_FLAG_PREP_DONE)) && (p.K == 64 || p.K == 128 || p.K == 256) &&
-         p.V % 64 == 0;
+         p.V % 64 == 0 && (long)p.B * p.H * (p.V / 64) < (1L << 31);
 }
 
 int token_step_fwd(const jla_problem& p, const jla_fwd_io& io, cudaStream_t s) {

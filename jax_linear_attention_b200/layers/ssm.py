@@ -74,7 +74,7 @@ def _step(x, dt, a, b, c, d, segment_ids, initial_state, output_final_state, chu
     groups, n = b.shape[2:]
     options = dict(initial_state=initial_state, segment_ids=segment_ids, chunk_size=chunk_size, precision=precision)
     b = ops.cuda.cast(b, c.dtype)
-    if (c.dtype != x.dtype or n not in (64, 128, 256) or width % 64 or precision == "chunked"
+    if (batch == 0 or c.dtype != x.dtype or n not in (64, 128, 256) or width % 64 or precision == "chunked"
             or (d is not None and d.shape != (heads,))
             or ops.cuda._reason("simple_gla", c, b, x, (dt,), options) is not None):
         return None

@@ -389,7 +389,7 @@ def _split_applies(kind, q, v, cu_seqlens, initial_state, precision) -> int:
 
 def _is_step(q, k, v, g, beta, initial_state, cu_seqlens, precision) -> bool:
     """A decoding step (one token per row and nothing to differentiate), which ``csrc/token_step.cu`` runs."""
-    return (q.shape[1] == 1 and cu_seqlens is None and _path(precision) != "chunked"
+    return (q.shape[1] == 1 and q.shape[0] > 0 and cu_seqlens is None and _path(precision) != "chunked"
             and not any(x is not None and x.requires_grad for x in (q, k, v, g, beta, initial_state)))
 
 

@@ -60,3 +60,21 @@ def test_ssd_step_matches_general_form(dtype, groups, skip):
     compare({"y": y.float().cpu().numpy(), "s": s.cpu().numpy()},
             {"y": y2.detach().float().cpu().numpy(), "s": s2.detach().cpu().numpy()},
             {"bfloat16": 2.0 ** -8, "float16": 2.0 ** -11}[dtype], "ssd step")
+
+
+def test_step_of_more_rows_than_a_grid_dimension_holds():
+    """65537 rows (gridDim.y ends at 65535): every row is its own step, so the last ones equal a call of their own."""
+    from jax_linear_attention_b200 import ops
+
+    gen = torch.Generator("cuda").manual_seed(9)
+    B, K, V = 65537, 64, 64
+    q, k, v = (torch.randn(B, 1, 1, 64, generator=gen, device="cuda").to(torch.bfloat16) for _ in range(3))
+    g = -torch.rand(B, 1, 1, generator=gen, device="cuda")
+    h0 = torch.randn(B, 1, K, V, generator=gen, device="cuda")
+    o, ht = ops.linear_attention("simple_gla", q, k, v, g=g, initial_state=h0, output_final_state=True)
+    tail = slice(B - 3, B)
+    o3, ht3 = ops.linear_attention("simple_gla", q[tail], k[tail], v[tail], g=g[tail], initial_state=h0[tail],
+                                   output_final_state=True)
+    assert torch.equal(o[tail], o3) and torch.equal(ht[tail], ht3)
+    want = torch.exp(g)[..., None] * h0 + k.float().transpose(-1, -2) * v.float()
+    assert torch.allclose(ht, want, rtol=1e-5, atol=1e-6)  # (one exp, one product and one sum in fp32)

@@ -55,3 +55,33 @@ def test_shared_prologue_belongs_to_its_queries(launches, monkeypatch, kind, V, 
             cuda._run(kind, x, k, v, g, beta, scale=1.0, initial_state=None, output_final_state=True, cu_seqlens=None,
                       segment_ids=None, use_qk_l2norm=l2norm)
     assert [done for done, _ in _prologues(launches)] == [False, True, False]
+
+
+def _step_inputs(B, H, Hk, K, V):
+    q, k = torch.empty(B, 1, Hk, K, dtype=torch.bfloat16), torch.empty(B, 1, Hk, K, dtype=torch.bfloat16)
+    return q, k, torch.empty(B, 1, H, V, dtype=torch.bfloat16), torch.empty(B, 1, H)
+
+
+@pytest.mark.parametrize("B", [0, 1, 65535, 65536])
+def test_decoding_steps_of_any_batch(launches, monkeypatch, B):
+    """A batch of any size runs: as one pass over the state from one row on, as the general call without rows."""
+    from jax_linear_attention_b200 import ops
+    from jax_linear_attention_b200.layers import mamba2_ssd
+
+    monkeypatch.setattr(torch.Tensor, "is_cuda", property(lambda self: True), raising=False)
+    lib = _lib.load()
+    for V in (256, 384, 512):  # wide value heads: the step kernel takes them whole
+        q, k, v, g = _step_inputs(B, 1, 1, 64, V)
+        ops.linear_attention("simple_gla", q, k, v, g=g)
+        p = launches[-1][1][0]
+        assert (p.B, p.H * p.V, p.V) == (B, V, V if B else 128)
+        assert lib.jla_fwd_scratch_bytes(p) == 0 if B else True
+        p.q = p.k = p.v = p.g = None
+        assert lib.jla_linear_attention_fwd(p, _lib.FwdIO(), None) == (_lib.ERR_BAD_ARGUMENT if B else _lib.OK)  # (no pointers)
+    launches.clear()
+    c, b, x, dt = _step_inputs(B, 1, 1, 64, 64)
+    mamba2_ssd(x, dt, torch.empty(1), b, c)
+    assert [name for name, _ in launches] == (["jla_ssd_step"] if B else ["jla_ssd_inputs_fwd", "jla_linear_attention_fwd"])
+    if B:
+        p = launches[0][1][0]
+        assert lib.jla_unsupported_reason(p) is None and lib.jla_fwd_scratch_bytes(p) == 0
