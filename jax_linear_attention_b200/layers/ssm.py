@@ -37,8 +37,8 @@ def mamba2_ssd(x, dt, a, b, c, *, d=None, segment_ids=None, initial_state=None, 
     if a.shape != (heads,):
         raise ValueError(f"a must be [H] = {(heads,)}; got {tuple(a.shape)}")
     if (x.shape[1] == 1 and x.is_cuda and x.dtype in _DTYPES and impl in ("auto", "cuda")
-            and not (torch.is_grad_enabled() and any(t is not None and t.requires_grad
-                                                     for t in (x, dt, a, b, c, d, initial_state)))):
+            and ops.is_builtin("simple_gla")
+            and ops.cuda.nothing_to_differentiate((x, dt, a, b, c, d, initial_state))):
         out = _step(x, dt, a, b, c, d, segment_ids, initial_state, output_final_state, chunk_size, precision)
         if out is not None:
             return out

@@ -59,6 +59,11 @@ for _kind in KINDS:
     register("cuda", _kind, cuda.FUNCTIONS[_kind], cuda.SUPPORTS[_kind], auto=True)
 
 
+def is_builtin(kind: str) -> bool:
+    """Whether ``kind`` still runs the kernels it was registered with here (a layer that fuses it with its own glue asks)."""
+    return _REGISTRY["cuda"].get(kind) == (cuda.FUNCTIONS[kind], cuda.SUPPORTS[kind], True)
+
+
 def linear_attention(kind: str, q, k, v, *, impl: str = "auto", **inputs: Any):
     """Run a linear-attention op; returns ``(o, final_state)``.
 

@@ -276,12 +276,26 @@ def _forward(q, k, v, g, beta, h0, k_read, cfg: dict, needs_grad: bool):
     return o, final, residuals, flags, rows
 
 
+def _no_transform() -> bool:
+    """No forward-mode level, no functorch transform, no tracer."""
+    return (torch.autograd.forward_ad._current_level < 0 and torch._C._functorch.peek_interpreter_stack() is None
+            and torch._C._get_tracing_state() is None and not torch.compiler.is_compiling())
+
+
 def _bypasses_autograd(tensors) -> bool:
     """Whether nothing could notice that a call does not go through ``torch.autograd.Function``: plain tensors of which
-    none requires a gradient, no forward-mode level, no functorch transform, no tracer."""
-    return (all(x is None or (not x.requires_grad and type(x) is torch.Tensor) for x in tensors)
-            and torch.autograd.forward_ad._current_level < 0 and torch._C._functorch.peek_interpreter_stack() is None
-            and torch._C._get_tracing_state() is None and not torch.compiler.is_compiling())
+    none requires a gradient, and no transform."""
+    return all(x is None or (not x.requires_grad and type(x) is torch.Tensor) for x in tensors) and _no_transform()
+
+
+_PLAIN = (torch.Tensor, torch.nn.Parameter, type(None))
+
+
+def nothing_to_differentiate(tensors) -> bool:
+    """The same for a layer around the op, which ``no_grad`` calls with parameters: plain tensors or parameters, no
+    transform, and gradients are off or none of them requires one."""
+    return (all(type(x) in _PLAIN for x in tensors) and _no_transform()
+            and not (torch.is_grad_enabled() and any(x is not None and x.requires_grad for x in tensors)))
 
 
 class _LinearAttention(torch.autograd.Function):

@@ -85,3 +85,41 @@ def test_decoding_steps_of_any_batch(launches, monkeypatch, B):
     if B:
         p = launches[0][1][0]
         assert lib.jla_unsupported_reason(p) is None and lib.jla_fwd_scratch_bytes(p) == 0
+
+
+def test_one_token_of_mamba2_is_a_step_only_where_nobody_could_tell(launches, monkeypatch):
+    """The fused step goes past autograd and past the table of implementations, so it leaves forward-mode tangents,
+    transforms, tensor subclasses and a replaced implementation to the general form; no_grad calls of parameters are steps."""
+    import torch.autograd.forward_ad as fwd
+
+    from jax_linear_attention_b200 import ops
+    from jax_linear_attention_b200.layers import mamba2_ssd
+
+    monkeypatch.setattr(torch.Tensor, "is_cuda", property(lambda self: True), raising=False)
+    c, b, x, dt = _step_inputs(2, 1, 1, 64, 64)
+    a = torch.nn.Parameter(-torch.ones(1))
+
+    def names(*args):
+        launches.clear()
+        mamba2_ssd(*args)
+        return [name for name, _ in launches]
+
+    general = ["jla_ssd_inputs_fwd", "jla_linear_attention_fwd"]
+    with torch.no_grad():
+        assert names(x, dt, a, b, c) == ["jla_ssd_step"]
+        assert names(x, dt, a, b.as_subclass(type("Labelled", (torch.Tensor,), {})), c) == general
+    assert names(x, dt, a, b, c) == general  # a requires a gradient
+    with fwd.dual_level():
+        with pytest.raises(NotImplementedError):  # as the general form has always answered
+            names(fwd.make_dual(x, torch.ones_like(x)), dt, a.detach(), b, c)
+        assert not any(name == "jla_ssd_step" for name, _ in launches)
+    with pytest.raises(RuntimeError):  # (the general form's autograd function has no rule for vmap)
+        torch.vmap(lambda x: mamba2_ssd(x, dt, a.detach(), b, c)[0])(x[None])
+    entry = ops._REGISTRY["cuda"]["simple_gla"]
+    calls = []
+    ops.register("cuda", "simple_gla", lambda *args, **kw: calls.append(kw) or entry[0](*args, **kw), entry[1], auto=True)
+    try:
+        assert names(x, dt, a.detach(), b, c) == general and len(calls) == 1
+    finally:
+        ops._REGISTRY["cuda"]["simple_gla"] = entry
+    assert names(x, dt, a.detach(), b, c) == ["jla_ssd_step"]
