@@ -461,6 +461,11 @@ class _PiecewiseContextParallel(torch.autograd.Function):
                 if has_h0:
                     s_in[0] = h0[0].to(sdt)
 
+            # inference tensors cannot enter a graph (nor can anything ask for their gradients)
+            if not any(ctx.needs_input_grad) and (torch.is_inference_mode_enabled() or any(x.is_inference() for x in xs)):
+                with torch.no_grad():
+                    o, f = pcall(kind, plain, cu_t, s_in)
+                return o, f[-1:].to(sdt)
             leaves = [x.detach().requires_grad_(True) for x in xs]
             s_in_leaf = s_in.requires_grad_(True)
             with torch.enable_grad():

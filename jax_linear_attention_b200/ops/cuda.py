@@ -223,6 +223,14 @@ class state_grads_only:
         _PassOptions.state_grads_only = self._outer
 
 
+def _identity(x):
+    """What makes ``x`` the same operand in two calls that keep it alive between them. Tensors of the inference mode have no
+    version to tell an update in place by: such a tensor equals nothing, itself included, so its tables are made again."""
+    if not isinstance(x, torch.Tensor):
+        return id(x)
+    return object() if x.is_inference() else (x.data_ptr(), x._version, x.shape, x.stride(), x.dtype)
+
+
 def _forward(q, k, v, g, beta, h0, k_read, cfg: dict, needs_grad: bool):
     """One forward launch: ``(o, final, residuals, flags, rows)``."""
     lib = _lib.load()
@@ -247,8 +255,7 @@ def _forward(q, k, v, g, beta, h0, k_read, cfg: dict, needs_grad: bool):
         # the way here). They are kept until the block ends, so their addresses stay theirs; a detached alias, which is how
         # the differentiated pass of a split gets its leaves, is the same memory at the same version.
         owners = cfg["prep_owners"]
-        identity = tuple((x.data_ptr(), x._version, x.shape, x.stride(), x.dtype) if isinstance(x, torch.Tensor) else id(x)
-                         for x in owners)
+        identity = tuple(_identity(x) for x in owners)
         key = (identity, tuple(q.shape), tuple(v.shape[2:3]), q.dtype, cfg["kind"], cfg["l2norm"],
                cfg["precision"])
         p.flags = flags | _lib.FLAG_SAVE_RESIDUALS

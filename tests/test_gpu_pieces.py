@@ -125,3 +125,20 @@ def test_pieces_of_narrow_values_keep_their_own_tables(kind, H, Hk):
                                                             torch.tensor(case["dht"], device="cuda", dtype=torch.float32)])
     got = {"o": o.detach(), "ht": ht.detach(), **{"d" + n: x for n, x in zip(t, grads)}}
     compare({n: x.float().cpu().numpy() for n, x in got.items()}, plain, 1e-2, f"{kind} pieces")
+
+
+def test_split_call_in_inference_mode(monkeypatch):
+    """Bit for bit the call under no_grad: the same kernels on the same operands."""
+    from jax_linear_attention_b200 import ops
+    from jax_linear_attention_b200.ops import cuda
+
+    monkeypatch.setattr(cuda, "MIN_SPLIT_CHUNKS", 8)
+    case = make_case("gated_deltanet", B=1, T=4096, H=4, K=128, V=128, seed=91, gates="baseline")
+    results = []
+    for mode in (torch.no_grad, torch.inference_mode):
+        with mode():
+            q, k, v = (torch.tensor(case[n], device="cuda", dtype=torch.bfloat16) for n in ("q", "k", "v"))
+            g, beta = (torch.tensor(case[n], device="cuda") for n in ("g", "beta"))
+            results.append(ops.linear_attention("gated_deltanet", q, k, v, g=g, beta=beta, output_final_state=True))
+    (o, ht), (o2, ht2) = results
+    assert torch.equal(o, o2) and torch.equal(ht, ht2)

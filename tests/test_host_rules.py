@@ -123,3 +123,22 @@ def test_one_token_of_mamba2_is_a_step_only_where_nobody_could_tell(launches, mo
     finally:
         ops._REGISTRY["cuda"]["simple_gla"] = entry
     assert names(x, dt, a.detach(), b, c) == ["jla_ssd_step"]
+
+
+def test_a_split_call_runs_in_inference_mode(launches, monkeypatch):
+    """The three passes of a split sequence on inference tensors: no graph, and every pass makes its own tables (such tensors
+    have no version that an update in place would change)."""
+    from jax_linear_attention_b200.distributed import context_parallel as cp
+
+    monkeypatch.setattr(torch.Tensor, "is_cuda", property(lambda self: True), raising=False)
+    monkeypatch.setattr(cp, "piece_scan", lambda *args, **kw: None)
+    with torch.inference_mode():
+        q, k, v = (torch.zeros(1, 1000, 2, 128, dtype=torch.bfloat16) for _ in range(3))
+        g, beta = torch.zeros(1, 1000, 2), torch.zeros(1, 1000, 2)
+    for mode in (torch.inference_mode, torch.no_grad):  # (inference tensors leave the mode as what they are)
+        launches.clear()
+        with mode():
+            o, ht = cp.context_parallel_linear_attention("gated_deltanet", q, k, v, g=g, beta=beta, group=False, piece_len=256,
+                                                         impl="cuda", output_final_state=True)
+        assert o.shape == v.shape and ht.shape == (1, 2, 128, 128) and not o.requires_grad
+        assert [done for done, _ in _prologues(launches)] == [False] * 3
