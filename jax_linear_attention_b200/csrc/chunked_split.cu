@@ -19,7 +19,10 @@
 // 150 us (fused 439 + 436); what bounds them now is the latency of a chunk's loads, barriers and products at one to four
 // CTAs of four warps an SM.
 //
-// Rounding is that of the fused kernels: 16-bit operands, fp32 accumulation, the carried state in fp32, Z in fp32.
+// 16-bit operands, fp32 accumulation, the carried state in fp32, Z in fp32. The reverse walk rounds the weighted query
+// fragments (the weighted dO once did); in f16 the weights are lifted to the chunk's largest one first, see state_kernel.
+#include <type_traits>
+
 #include "chunked.cuh"
 #include "profile.cuh"
 #include "mma.cuh"
@@ -63,6 +66,10 @@ __global__ void __launch_bounds__(NT) state_kernel(StateParams p) {
   constexpr int LDK = L::LDK, LDV = L::LDV, LDC = L::LDC;
   constexpr int NTV = VB / 8;   // n-tiles across the value columns
   constexpr int MT = K / 64;    // 16-row tiles of the state per warp
+  // f16 backward: the weights scale (cin Gamma) of a chunk that starts behind a strong decay would push the weighted query
+  // fragments below the type's normal range (unit rows behind e^-8: the chunk's share of dS off by 8e-3). They are carried
+  // relative to the power of two above the largest one, which the fp32 accumulators take out again.
+  constexpr bool kLift = BWD && std::is_same<T, __half>::value;
   const int vblocks = p.V / VB;
   const int v0 = (blockIdx.x % vblocks) * VB, rh = blockIdx.x / vblocks;
   const int row = rh / p.H, h = rh - row * p.H, hk = h / (p.H / p.Hk);
@@ -147,9 +154,16 @@ __global__ void __launch_bounds__(NT) state_kernel(StateParams p) {
     T* hout = static_cast<T*>(p.h) + ((long)c * p.H + h) * K * p.V + v0;
     // the per-token weight of the update that is applied to the key or query fragments, in the (here unused) beta half
     // of the gate vectors: tail Gamma_r forward, scale (cin Gamma) backward; a barrier follows before its readers
+    float lift = 1.f, unlift = 1.f;
+    if (kLift) {
+      const float a = p.scale * row_scalars(Gs, runs, m.flags, lane).gam;
+      const float b = p.scale * row_scalars(Gs, runs, m.flags, lane + 32).gam;
+      const unsigned e = __reduce_max_sync(0xffffffffu, __float_as_uint(fmaxf(fabsf(a), fabsf(b)))) >> 23;
+      if (e > 0 && e < 253) lift = __uint_as_float((253 - e) << 23), unlift = __uint_as_float((e + 1) << 23);
+    }
     if ((BWD || !DELTA) && tid < 64) {
       const RowScalars r = row_scalars(Gs, runs, m.flags, tid);
-      stage_g(s)[64 + tid] = BWD ? p.scale * r.gam : r.gamr;
+      stage_g(s)[64 + tid] = BWD ? p.scale * r.gam * lift : r.gamr;
     }
     if (DELTA) {
       store_tile<T, VB>(hout, p.V, Sb, LDV, K, tid, NT);
@@ -204,7 +218,7 @@ __global__ void __launch_bounds__(NT) state_kernel(StateParams p) {
 #pragma unroll
       for (int nt = 0; nt < NTV; ++nt) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) acc[mt][nt][e] *= kg;
+        for (int e = 0; e < 4; ++e) acc[mt][nt][e] *= kg * lift;
       }
       const int a0 = sr0 + 16 * mt;
       if (!DELTA) {
@@ -214,6 +228,11 @@ __global__ void __launch_bounds__(NT) state_kernel(StateParams p) {
       } else {
         // Q^T (scale cin Gamma dO): needs nothing of the chain, ahead of the barrier the last product waits for
         warp_gemm_scaled_a<T, NTV, 4, B_KN>(acc[mt], stage_q(s) + a0, LDK, Gs + 64, stage_x(s), LDV, lane);
+      }
+#pragma unroll
+      for (int nt = 0; nt < (kLift ? NTV : 0); ++nt) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[mt][nt][e] *= unlift;
       }
     }
     if (DELTA && BWD) {

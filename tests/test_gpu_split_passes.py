@@ -7,7 +7,7 @@ import pytest
 import torch
 
 from oracle.cases import make_case
-from tests._util import compare, run_cuda
+from tests._util import compare, run_cuda, run_oracle
 
 pytestmark = pytest.mark.gpu
 
@@ -27,3 +27,24 @@ def test_split_passes_match_the_scan(kind, B, T, H, Hk, K, V, dtype):
     want = run_cuda(kind, case, scale=case["meta"]["scale"], dtype=dtype, precision="highest")
     got = run_cuda(kind, case, scale=case["meta"]["scale"], dtype=dtype)
     compare(got, want, {"bfloat16": 1e-2, "float16": 2e-3}[dtype], f"{kind} B{B} T{T} H{H} K{K} V{V}")
+
+
+@pytest.mark.parametrize("kind,dO", [("gated_deltanet", 1.0), ("gated_deltanet", 1e-3), ("simple_gla", 1.0)])
+def test_float16_state_gradient_behind_a_strong_decay(kind, dO):
+    """A chunk that starts behind e^-8: what its queries send back to the entering state is that factor times a sum of 64
+    products, every factor of them a normal f16 number (unit rows / 8, upstream gradients of 1 and of 1e-3). So dh0 is off
+    by the rounding of the weighted operand (2^-11 an element, averaged over the sum); without writes (beta = 0) nothing
+    else reaches it."""
+    import numpy as np
+
+    case = make_case(kind, B=2, T=64, H=2, K=64, V=64, seed=5, dtype="float16", h0=True)
+    case["q"] = case["q"] / 4  # rows of length 4 otherwise
+    case["g"] = np.full_like(case["g"], -0.01)
+    case["g"][:, 0] = -8.0
+    if "beta" in case:
+        case["beta"] = np.zeros_like(case["beta"])
+    case["dht"] = np.zeros_like(case["dht"])
+    case["do"] = (case["do"] * dO).astype(np.float16).astype(np.float32)
+    want = run_oracle(kind, case, scale=case["meta"]["scale"])
+    got = run_cuda(kind, case, scale=case["meta"]["scale"], dtype="float16")
+    compare({"dh0": got["dh0"]}, {"dh0": want["dh0"]}, 2.0 ** -11, f"{kind} {dO}")
