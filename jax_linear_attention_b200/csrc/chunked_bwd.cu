@@ -11,6 +11,8 @@
 // second, transposed products).
 #include <stdlib.h>
 
+#include <type_traits>
+
 #include "chunked.cuh"
 #include "profile.cuh"
 #include "mma.cuh"
@@ -657,12 +659,32 @@ __global__ void __launch_bounds__(512, 1) decay_grads_kernel(BwdParams p) {
     }
   }
 
-  __syncthreads();  // every head's terms are complete, P is free
+  // The sum of the heads' dP tiles may leave the range of f16 where each of them is inside: their mean is taken then.
+  bool over = false;
+  if (NH > 1 && std::is_same<T, __half>::value) {
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) over |= !(fabsf(sumP[nt][e]) <= 65504.f);
+    }
+  }
+  over = __syncthreads_or(over);  // every head's terms are complete, P is free
+  auto scale_acc = [&](float x) {
+#pragma unroll
+    for (int nt = 0; nt < KNT; ++nt) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[nt][e] *= x;
+    }
+  };
+  constexpr float kMean = 1.f / NH;
+  const float share = over ? kMean : 1.f;
   if (p.dg && tid < 32) write_dg(NH - 1);
-  if (!keys) store_acc<T, 4>(P0, LDC, r0, cc0, sumP, lane);
+  if (!keys) store_acc<T, 4>(P0, LDC, r0, cc0, sumP, lane, share, share);
+  if (over) scale_acc(kMean);
   __syncthreads();
   if (!keys) warp_gemm<T, KNT, 4, A_ROW, B_KN>(acc, P0 + r0 * LDC, LDC, kS + kc0, LDK, lane);
   else warp_gemm<T, KNT, 4, A_COL, B_KN>(acc, P0 + r0, LDC, qS + kc0, LDK, lane);
+  if (over) scale_acc(NH);
   float* sums = keys ? p.dk_acc : p.dq_acc;
   T* direct = static_cast<T*>(keys ? p.dk : p.dq);
 #pragma unroll

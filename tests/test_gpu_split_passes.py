@@ -48,3 +48,21 @@ def test_float16_state_gradient_behind_a_strong_decay(kind, dO):
     want = run_oracle(kind, case, scale=case["meta"]["scale"])
     got = run_cuda(kind, case, scale=case["meta"]["scale"], dtype="float16")
     compare({"dh0": got["dh0"]}, {"dh0": want["dh0"]}, 2.0 ** -11, f"{kind} {dO}")
+
+
+@pytest.mark.parametrize("H,Hk,K", [(8, 1, 128), (8, 2, 64)])
+def test_float16_head_sums_beyond_the_range_of_one_head(H, Hk, K):
+    """Upstream gradients of one sign over a group of heads: each head's dP stays inside f16 (64 * 1 * 300 = 19200), their sum
+    does not. dq and dk, which are small because the keys and queries are, come out as of the fp32 scan. (So small queries and
+    keys make o and the in-chunk part of dv subnormal f16 numbers: those two are only held to be finite.)"""
+    import numpy as np
+
+    case = make_case("simple_gla", B=1, T=130, H=H, Hk=Hk, K=K, V=64, seed=6, dtype="float16", h0=True)
+    case["q"], case["k"] = case["q"] / 256, case["k"] / 256
+    case["v"], case["do"] = np.ones_like(case["v"]), np.full_like(case["do"], 300.0)
+    case["g"] = np.full_like(case["g"], -0.01)
+    case["h0"], case["dht"] = case["h0"] / 256, case["dht"] / 256
+    want = run_cuda("simple_gla", case, scale=1.0, dtype="float16", precision="highest")
+    got = run_cuda("simple_gla", case, scale=1.0, dtype="float16")
+    assert all(np.isfinite(x).all() for x in got.values())
+    compare(got, {n: x for n, x in want.items() if n not in ("o", "dv")}, 2e-3, f"{H} {Hk} {K}")
