@@ -27,7 +27,7 @@ struct Plan {
   bool delta, l2norm, save;
   size_t meta, row_chunks, gates, runs, t0, ag, qn, kn, h, vn, w, residual_bytes;  // residual buffer
   size_t kda_q, kda_kr, kda_kw, kda_p, kda_d;  // KDA: gate-folded operands per chunk slot (see chunked_kda_prep.cu)
-  size_t qk_tab;  // grouped simple GLA on the mma.sync kernels: Q K^T and K Q^T per (chunk, key head), see qk_table_kernel
+  size_t qk_tab;  // grouped simple GLA on the mma.sync kernels: Q K^T per (chunk, key head), see qk_table_kernel
   size_t z;  // backward of the split kernels: scale P^T dO in fp32, see chunked_split.cu
   size_t kda_dag, kda_dqs, kda_dks, kda_dku, kda_dd;  // KDA backward scratch (see chunked_kda_bwd.cu)
   size_t fwd_scratch_bytes;                                                 // same layout without h, vn
@@ -52,10 +52,10 @@ template <>
 __host__ __device__ constexpr float kda_bounded_log<__half>() { return 12.f; }
 
 // Without the delta rule the in-chunk scores Q K^T do not depend on the value head: when several value heads share a
-// key head (Mamba-2: all of them) the mma.sync kernels take the two 64 x 64 products Q K^T and K Q^T from a table
-// that a small kernel fills once per (chunk, key head), in the accumulator-fragment order of the warps that use
-// them (fp32, so the decayed scores round exactly as when every head computes the product itself).
-constexpr int kQkTabFloats = 2 * 64 * 64;  // per (chunk, key head): Q K^T then K Q^T
+// key head (Mamba-2: all of them) the fused forward and the gradient kernel's walks over heads take the 64 x 64 product
+// from a table that a small kernel fills once per (chunk, key head), in the accumulator-fragment order of the warps that
+// use it (fp32, so the decayed scores round exactly as when every head computes the product itself).
+constexpr int kQkTabFloats = 64 * 64;  // per (chunk, key head)
 inline bool shares_scores(const jla_problem& p) {
   return p.kind == JLA_KIND_SIMPLE_GLA && !use_tc_kernels(p) && p.Hk > 0 && p.H / p.Hk >= 2;
 }

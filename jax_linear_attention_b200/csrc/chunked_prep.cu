@@ -235,10 +235,10 @@ int launch_kkt(const KktParams& kp, int blocks, cudaStream_t s) {
   return JLA_OK;
 }
 
-// Q K^T and K Q^T of one (chunk, key head) in fp32, stored in the accumulator-fragment order of warp_gemm: for the row
-// block rb = warp (16 rows), fragment register i (0 .. 31 = n-tile * 4 + e) of lane l sits at ((rb * 8 + i / 4) * 32 + l)
-// * 4 + i % 4, so that a warp of the state-pass kernels reads its whole 16 x 64 block with eight coalesced 16-byte
-// loads per lane. The products are the same instruction sequence the kernels would otherwise run per value head.
+// Q K^T of one (chunk, key head) in fp32, stored in the accumulator-fragment order of warp_gemm: for the row block
+// rb = warp (16 rows), fragment register i (0 .. 31 = n-tile * 4 + e) of lane l sits at ((rb * 8 + i / 4) * 32 + l) * 4
+// + i % 4, so that a warp of the kernels that use it reads its whole 16 x 64 block with eight coalesced 16-byte loads per
+// lane. The product is the same instruction sequence the kernels would otherwise run per value head.
 template <typename T, int K>
 __global__ void __launch_bounds__(128) qk_table_kernel(const ChunkMeta* meta, const void* q, const void* k, float* tab, int Hk) {
   constexpr int LDK = K + 8;
@@ -254,16 +254,12 @@ __global__ void __launch_bounds__(128) qk_table_kernel(const ChunkMeta* meta, co
   cp_async_commit();
   cp_async_wait<0>();
   __syncthreads();
-  float* out = tab + (long)blockIdx.x * kQkTabFloats;
+  float acc[8][4];
+  zero_acc(acc);
+  warp_gemm<T, 8, K / 16, A_ROW, B_NK>(acc, qS + 16 * warp * LDK, LDK, kS, LDK, lane);
+  float4* dst = reinterpret_cast<float4*>(tab + (long)blockIdx.x * kQkTabFloats) + warp * 8 * 32 + lane;
 #pragma unroll
-  for (int variant = 0; variant < 2; ++variant) {
-    float acc[8][4];
-    zero_acc(acc);
-    warp_gemm<T, 8, K / 16, A_ROW, B_NK>(acc, (variant ? kS : qS) + 16 * warp * LDK, LDK, variant ? qS : kS, LDK, lane);
-    float4* dst = reinterpret_cast<float4*>(out + variant * 4096) + warp * 8 * 32 + lane;
-#pragma unroll
-    for (int nt = 0; nt < 8; ++nt) dst[nt * 32] = make_float4(acc[nt][0], acc[nt][1], acc[nt][2], acc[nt][3]);
-  }
+  for (int nt = 0; nt < 8; ++nt) dst[nt * 32] = make_float4(acc[nt][0], acc[nt][1], acc[nt][2], acc[nt][3]);
 }
 
 template <typename T>
