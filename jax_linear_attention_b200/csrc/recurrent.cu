@@ -41,6 +41,7 @@ constexpr int VTS = VT + 4;   // (stride of a staged state row: 16-byte reads of
 struct RecParams {
   Rows rows;
   int H, Hk, K, V;
+  int head0, heads;  // the value heads of this launch
   int gate;  // 0 none, 1 scalar, 2 per key channel
   int delta, l2norm;
   float scale;
@@ -55,7 +56,7 @@ struct RecParams {
   float* dkr_acc;          // [B*T, H, K] f32: gradient of k_read (with k_read only)
   void* dv;
   float *dg, *dbeta, *dh0;
-  // [H][slots][K*V]: the state entering every block of a row; the state gradient coming from behind every block. Slot of
+  // [heads][slots][K*V]: the state entering every block of a row; the state gradient coming from behind every block. Slot of
   // block b of a row: slot0(row) + b.
   float *s_ckpt, *ds_ckpt;
   float *resid, *du;  // [B*T, H, V] f32: v_t - r_t and the gradient of the written value u_t
@@ -270,8 +271,8 @@ __device__ __forceinline__ void forward_walk(const RecParams& p, WalkSmem<KL>& s
   float* ckpt = nullptr;
   if (!OP) {
     const long slot = p.slot0(r, tok0);
-    ckpt = p.s_ckpt + ((long)h * p.slots + slot) * K * V;
-    if (h == 0 && v0 == 0) {
+    ckpt = p.s_ckpt + ((long)(h - p.head0) * p.slots + slot) * K * V;
+    if (h == p.head0 && v0 == 0) {
       for (int b = threadIdx.x; b * TB < len; b += NW * 32) p.slot_row[slot + b] = r;
     }
   }
@@ -350,7 +351,7 @@ __device__ __forceinline__ void reverse_walk(const RecParams& p, WalkSmem<KL>& s
   const Lane<KL> me(v0, V);
   Chan dS;
   me.load_state(p.d_final ? p.d_final + ((long)r * p.H + h) * K * V : nullptr, K, V, dS);
-  float* ckpt = p.ds_ckpt + ((long)h * p.slots + p.slot0(r, tok0)) * K * V;
+  float* ckpt = p.ds_ckpt + ((long)(h - p.head0) * p.slots + p.slot0(r, tok0)) * K * V;
   const float(*read_key)[WalkSmem<KL>::KP] = p.k_read ? s.kr : s.k;
   Stage<T, KL> st;
   const int last = len > 0 ? (len - 1) / SB * SB : -SB;
@@ -404,19 +405,19 @@ __device__ __forceinline__ void reverse_walk(const RecParams& p, WalkSmem<KL>& s
   if (p.dh0) me.store_state(p.dh0 + ((long)r * p.H + h) * K * V, K, V, dS);
 }
 
-// grid: (H * column blocks, rows)
+// grid: (heads * column blocks, rows)
 template <typename T, int KL, int MODE>
 __global__ void __launch_bounds__(NW * 32) rec_fwd_kernel(RecParams p) {
   __shared__ __align__(16) WalkSmem<KL> s;
-  const int h = blockIdx.x % p.H, v0 = blockIdx.x / p.H * WalkSmem<KL>::NC;
+  const int h = p.head0 + blockIdx.x % p.heads, v0 = blockIdx.x / p.heads * WalkSmem<KL>::NC;
   forward_walk<T, KL, MODE, true>(p, s, blockIdx.y, h, v0);
 }
 
-// grid: (2 * H * column blocks, rows); the two walks are independent of each other
+// grid: (2 * heads * column blocks, rows); the two walks are independent of each other
 template <typename T, int KL, int MODE>
 __global__ void __launch_bounds__(NW * 32) rec_bwd_kernel(RecParams p) {
   __shared__ __align__(16) WalkSmem<KL> s;
-  const int x = blockIdx.x >> 1, h = x % p.H, v0 = x / p.H * WalkSmem<KL>::NC;
+  const int x = blockIdx.x >> 1, h = p.head0 + x % p.heads, v0 = x / p.heads * WalkSmem<KL>::NC;
   if (blockIdx.x & 1) reverse_walk<T, KL, MODE>(p, s, blockIdx.y, h, v0);
   else forward_walk<T, KL, MODE, false>(p, s, blockIdx.y, h, v0);
 }
@@ -461,8 +462,8 @@ template <typename T>
 __global__ void __launch_bounds__(GT) block_grads_kernel(RecParams p) {
   extern __shared__ __align__(16) float smem_raw[];
   const int K = p.K, V = p.V, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int h = blockIdx.x % p.H, hk = h / (p.H / p.Hk);
-  const long slot = blockIdx.x / p.H;
+  const int hl = blockIdx.x % p.heads, h = p.head0 + hl, hk = h / (p.H / p.Hk);
+  const long slot = blockIdx.x / p.heads;
   const int row = p.slot_row[slot];
   if (row < 0 || row >= p.rows.count()) return;
   int tok0, len;
@@ -551,8 +552,8 @@ __global__ void __launch_bounds__(GT) block_grads_kernel(RecParams p) {
     s.urt[t * TB + j] = s.ur[tid] = ct;
   }
 
-  const float* S0 = p.s_ckpt + ((long)h * p.slots + slot) * K * V;
-  const float* dE = p.ds_ckpt + ((long)h * p.slots + slot) * K * V;
+  const float* S0 = p.s_ckpt + ((long)hl * p.slots + slot) * K * V;
+  const float* dE = p.ds_ckpt + ((long)hl * p.slots + slot) * K * V;
   const int cl = tid % CT, tg = tid / CT, tq = 4 * tg;  // channel of the tile; this thread's tokens are tq .. tq + 3
   double gsum = 0.;                                     // scalar gates: a sixteenth of dg of token tid / 16
   for (int c0 = 0; c0 < K; c0 += CT) {
@@ -724,6 +725,7 @@ RecParams base_params(const jla_problem& p) {
   RecParams r{};
   r.rows = make_rows(p);
   r.H = p.H; r.Hk = p.Hk; r.K = p.K; r.V = p.V;
+  r.head0 = 0; r.heads = p.H;
   r.gate = p.kind == JLA_KIND_DELTANET ? 0 : (p.kind == JLA_KIND_KDA ? 2 : 1);
   r.delta = p.kind != JLA_KIND_SIMPLE_GLA;
   r.l2norm = (p.flags & JLA_FLAG_QK_L2NORM) != 0;
@@ -737,7 +739,7 @@ template <typename T, int KL>
 int launch_walks(const RecParams& rp, bool bwd, int rows, cudaStream_t stream) {
   const int blocks = (rp.V + WalkSmem<KL>::NC - 1) / WalkSmem<KL>::NC;
   ProfScope ps(bwd ? kProfRecBwd : kProfRecFwd, stream);
-  const dim3 grid((unsigned)(rp.H * blocks * (bwd ? 2 : 1)), (unsigned)rows);
+  const dim3 grid((unsigned)(rp.heads * blocks * (bwd ? 2 : 1)), (unsigned)rows);
   auto run = [&](auto* fwd, auto* back) { (bwd ? back : fwd)<<<grid, NW * 32, 0, stream>>>(rp); };
   if (!rp.delta) run(rec_fwd_kernel<T, KL, kHeadDecay>, rec_bwd_kernel<T, KL, kHeadDecay>);
   else if (rp.gate == 2) run(rec_fwd_kernel<T, KL, kChannelDelta>, rec_bwd_kernel<T, KL, kChannelDelta>);
@@ -759,7 +761,7 @@ int launch_t(const RecParams& rp, bool bwd, int rows, cudaStream_t stream) {
   const size_t smem = GradSmem::floats(rp.K, rp.V) * sizeof(float);
   JLA_CUDA_OK(cudaFuncSetAttribute(block_grads_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   ProfScope ps(kProfRecGrads, stream);
-  block_grads_kernel<T><<<(unsigned)(rp.slots * rp.H), GT, smem, stream>>>(rp);
+  block_grads_kernel<T><<<(unsigned)(rp.slots * rp.heads), GT, smem, stream>>>(rp);
   JLA_LAUNCH_OK();
   return JLA_OK;
 }
@@ -778,8 +780,15 @@ struct BwdScratch {
   float *dq_acc, *dk_acc, *dkr_acc, *s_ckpt, *ds_ckpt, *resid, *du;
   int* slot_row;
   long slots;
+  int heads;
   size_t bytes;
 };
+
+// The two checkpoint sets take K V / 2 bytes a token and head (twice what one walk with one set took, eight kilobytes at
+// K = V = 128), so very long calls run a slice of the heads at a time through the same buffers: heads are independent, and
+// the slices follow each other on the stream. The limit leaves a call of 180 GB the room that it had with one set, and
+// sends no call of ordinary size through slices, which are walks one after the other.
+constexpr size_t kMaxCheckpointBytes = 32ull << 30;
 
 BwdScratch carve_bwd(const jla_problem& p, void* base) {
   Carver c(base);
@@ -791,8 +800,12 @@ BwdScratch carve_bwd(const jla_problem& p, void* base) {
   s.dq_acc = c.take<float>((size_t)tokens * p.H * p.K);
   s.dk_acc = c.take<float>((size_t)tokens * p.H * p.K);
   s.dkr_acc = c.take<float>(p.k_read ? (size_t)tokens * p.H * p.K : 0);
-  s.s_ckpt = c.take<float>((size_t)p.H * s.slots * p.K * p.V);
-  s.ds_ckpt = c.take<float>((size_t)p.H * s.slots * p.K * p.V);
+  const size_t per_head = (size_t)s.slots * p.K * p.V;  // of one set, in floats
+  const size_t fit = kMaxCheckpointBytes / (2 * sizeof(float) * per_head);
+  const int slices = fit >= (size_t)p.H ? 1 : fit > 0 ? (int)((p.H + fit - 1) / fit) : p.H;
+  s.heads = (p.H + slices - 1) / slices;
+  s.s_ckpt = c.take<float>(s.heads * per_head);
+  s.ds_ckpt = c.take<float>(s.heads * per_head);
   s.resid = c.take<float>(delta ? (size_t)tokens * p.H * p.V : 0);
   s.du = c.take<float>(delta ? (size_t)tokens * p.H * p.V : 0);
   s.slot_row = c.take<int>((size_t)s.slots);
@@ -834,7 +847,8 @@ int recurrent_bwd(const jla_problem& p, const jla_bwd_io& io, cudaStream_t strea
   rp.slot_row = s.slot_row; rp.slots = s.slots;
   const int rows = p.cu_seqlens ? p.num_seqs : p.B;
   const long tokens = (long)p.B * p.T;
-  if (rows > 0 && p.H > 0) {
+  for (rp.head0 = 0; rows > 0 && rp.head0 < p.H; rp.head0 += s.heads) {
+    rp.heads = p.H - rp.head0 < s.heads ? p.H - rp.head0 : s.heads;
     const int rc = launch_dtype(rp, p.dtype, true, rows, stream);
     if (rc != JLA_OK) return rc;
   }

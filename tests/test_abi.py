@@ -70,6 +70,26 @@ def test_unsupported_reason_and_sizes_without_a_gpu():
     assert rc == _lib.ERR_BAD_ARGUMENT and b"batch size 1" in lib.jla_last_error()
 
 
+def test_token_scan_scratch_is_bounded_for_very_long_calls():
+    """The backward's checkpoints (two states every 16 tokens of a row) take at most 32 GiB, or one head's share of it."""
+    from jax_linear_attention_b200 import _lib
+
+    lib = _lib.load()
+    p = _lib.Problem()
+    p.kind, p.dtype, p.path, p.flags = _lib.KIND["gated_deltanet"], 2, 0, _lib.FLAG_SAVE_RESIDUALS
+    p.num_seqs, p.scale, p.K, p.V = 0, 1.0, 128, 128
+
+    def checkpoints(T, H):
+        p.B, p.T, p.H, p.Hk = 1, T, H, H
+        vectors = 4 * 4 * T * H * 128  # dq, dk, v - r, du
+        return lib.jla_bwd_scratch_bytes(ctypes.byref(p)) - vectors
+
+    per_head = 2 * 4 * 128 * 128
+    assert checkpoints(4096, 16) >= 256 * 16 * per_head  # all heads at once
+    assert 2 ** 34 <= checkpoints(1 << 20, 16) <= 2 ** 35 + 2 ** 20 * 16
+    assert checkpoints(1 << 24, 2) <= (2 ** 20 + 2) * per_head + 2 ** 27
+
+
 @pytest.mark.parametrize("kind,K,V", [("gated_deltanet", 256, 512), ("simple_gla", 128, 192), ("kda", 128, 512)])
 def test_a_decoding_step_has_no_backward(kind, K, V):
     """Head sizes that only the decoding-step kernel covers: the forward is accepted, nothing of a backward is."""

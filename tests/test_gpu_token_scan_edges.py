@@ -5,6 +5,7 @@ per tensor stays around 2e-7 (2^-24 per operation, sums of a few hundred terms),
 
 import numpy as np
 import pytest
+import torch
 
 from oracle.cases import make_case
 from tests._util import compare, run_cuda, run_oracle
@@ -51,3 +52,27 @@ def test_gate_gradients_entry_by_entry_behind_strong_decays(kind):
     assert (got["dg"][:, 0] == 0).all()
     err = np.abs(got["dg"][:, 1:] - want["dg"][:, 1:]) / np.abs(want["dg"][:, 1:])
     assert np.median(err) < 2e-6, np.median(err)
+
+
+def test_heads_in_slices_are_the_heads_of_calls_of_their_own():
+    """Checkpoints of more than 32 GiB: 33 heads of 256 x 256 over 1024 rows run as slices of 17 and 16 heads through the same
+    buffers, with the results of two calls of 17 and 16 heads, bit for bit."""
+    from jax_linear_attention_b200 import ops
+
+    gen = torch.Generator("cuda").manual_seed(4)
+    B, T, H, K = 1024, 16, 33, 256
+
+    def normal(*shape):
+        return torch.randn(*shape, generator=gen, device="cuda") / 16
+
+    x = [normal(B, T, H, K) for _ in range(3)] + [-normal(B, T, H).abs(), torch.sigmoid(normal(B, T, H))]
+    do = normal(B, T, H, K)
+
+    def gradients(heads):
+        leaves = [t[:, :, heads].contiguous().requires_grad_(True) for t in x]
+        o, _ = ops.linear_attention("gated_deltanet", *leaves[:3], g=leaves[3], beta=leaves[4], scale=1.0)
+        return torch.autograd.grad(o, leaves, do[:, :, heads])
+
+    parts = [torch.cat(p, 2) for p in zip(gradients(slice(0, 17)), gradients(slice(17, 33)))]
+    for whole, part in zip(gradients(slice(0, 33)), parts):
+        assert torch.equal(whole, part)
