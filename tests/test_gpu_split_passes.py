@@ -7,7 +7,8 @@ import pytest
 import torch
 
 from oracle.cases import make_case
-from tests._util import compare, run_cuda, run_oracle
+from jax_linear_attention_b200 import _lib
+from tests._util import cabi_fwd_bwd, compare, run_cuda, run_oracle
 
 pytestmark = pytest.mark.gpu
 
@@ -66,3 +67,38 @@ def test_float16_head_sums_beyond_the_range_of_one_head(H, Hk, K):
     got = run_cuda("simple_gla", case, scale=1.0, dtype="float16")
     assert all(np.isfinite(x).all() for x in got.values())
     compare(got, {n: x for n, x in want.items() if n not in ("o", "dv")}, 2e-3, f"{H} {Hk} {K}")
+
+
+@pytest.mark.parametrize("H,Hk,K,dtype", [(16, 2, 64, "bfloat16"), (8, 2, 64, "float16"), (6, 3, 64, "bfloat16"),
+                                          (4, 2, 128, "float16"), (3, 1, 64, "bfloat16")])
+def test_walks_over_eight_four_two_and_one_heads_of_a_group(H, Hk, K, dtype):
+    """The gradients without the delta rule, for every length of a walk over the heads of a key group and both key sizes."""
+    case = make_case("simple_gla", B=2, T=130, H=H, Hk=Hk, K=K, V=64, seed=H + K, dtype=dtype, docs="mixed", h0=True)
+    want = run_cuda("simple_gla", case, scale=case["meta"]["scale"], dtype=dtype, precision="highest")
+    got = run_cuda("simple_gla", case, scale=case["meta"]["scale"], dtype=dtype)
+    compare(got, want, {"bfloat16": 1e-2, "float16": 2e-3}[dtype], f"{H} {Hk} {K}")
+
+
+@pytest.mark.parametrize("kind", ["simple_gla", "kda"])
+def test_outputs_that_are_not_16_byte_aligned(kind):
+    """Where the kernels store 16 bytes out of their accumulators, a buffer at an odd multiple of four bytes takes the narrow
+    stores: the same values (dv of the split kernels, dq and dk of KDA's)."""
+    K, V = (128, 64) if kind == "simple_gla" else (128, 128)
+    case = make_case(kind, B=2, T=100, H=2, K=K, V=V, seed=12, dtype="bfloat16", docs="mixed",
+                     gates="kda_baseline" if kind == "kda" else "baseline")
+    out = cabi_fwd_bwd(kind, case, scale=case["meta"]["scale"])
+    t, p, dev = out["tensors"], out["problem"], out["o"].device
+
+    def buffer(like, shift):  # `shift` elements behind a 16-byte boundary
+        return torch.empty(like.numel() + 8, dtype=like.dtype, device=dev)[shift:][:like.numel()].view(like.shape)
+
+    got = {n: buffer(out[n], 2 if n in (("dv",) if kind == "simple_gla" else ("dq", "dk")) else 0)
+           for n in ("dq", "dk", "dv", "dg", "dbeta", "dh0") if out[n] is not None}
+    assert any(x.data_ptr() % 16 == 4 for x in got.values())
+    scratch = torch.empty_like(out["bwd_scratch"])
+    io = _lib.BwdIO(t["do"].data_ptr(), t["dht"].data_ptr() if "dht" in t else None,
+                    *(got[n].data_ptr() if n in got else None for n in ("dq", "dk", "dv", "dg", "dbeta", "dh0")),
+                    out["residuals"].data_ptr(), out["residuals"].numel(), scratch.data_ptr(), scratch.numel())
+    _lib.launch("jla_linear_attention_bwd", dev, p, io)
+    for name, x in got.items():
+        assert torch.equal(x, out[name]), name
