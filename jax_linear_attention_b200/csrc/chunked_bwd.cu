@@ -426,10 +426,11 @@ __global__ void __launch_bounds__(256, 1) sg_chunk_grads_kernel(BwdParams p) {
 //
 // Sixteen warps in two groups of eight: the query group forms P, dP and the dq terms, the key group the dk terms, <S, dS+>
 // and dV (for which it takes P from the query group). Bound by the latency of its dependent instructions at four warps a
-// scheduler (0.3 issued a cycle, tensor pipe 15 %). Measured at B8 T2048 H64 P64 N128: 588 us; with the score table read from
-// L2 for every head and the document test in every element 674 us; with <S, dS+> in the query group as well 768 us; as one group of eight warps, two CTAs an SM, both accumulators in every warp (spilling) 709 us; the form
-// with a product with K and one with Q per head, and dV in a kernel of its own, 613 + 149 us. The tiles of the next head
-// are on their way for the whole time of one head: one block-wide barrier a head, and a hand-over of P between the groups.
+// scheduler (0.3 issued a cycle, tensor pipe 15 %). Measured at B8 T2048 H64 P64 N128: 588 us; with the score table read
+// from L2 for every head and the document test in every element 674 us; with <S, dS+> in the query group as well 768 us; as
+// one group of eight warps, two CTAs an SM, both accumulators in every warp (spilling) 709 us; the form with a product with
+// K and one with Q per head, and dV in a kernel of its own, 613 + 149 us. The tiles of the next head are on their way for
+// the whole time of one head: one block-wide barrier a head, and a hand-over of P between the groups.
 template <typename T, int K, int V>
 struct DecayGradSmem {
   static constexpr int LDK = K + 8, LDV = V + 8, LDC = 72;

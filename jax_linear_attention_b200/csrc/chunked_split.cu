@@ -287,8 +287,9 @@ struct TokenSmem {
   static_assert(NH == 1 || kStageElems <= 2 * 64 * LDK, "the second stage lies over the key tiles");
 };
 
-// Four warps, 16 rows each. NH > 1: the CTA walks NH adjacent value heads of one key head, for which the raw scores are
-// the same products: they stay in registers (as do a warp's rows of the state product's left operand), and the next head's tiles are on their way while one is worked on.
+// Four warps, 16 rows each. NH > 1: the CTA walks NH adjacent value heads of one key head, for which the raw scores are the
+// same products: they stay in registers (as do a warp's rows of the state product's left operand), and the next head's
+// tiles are on their way while one is worked on.
 template <typename T, int K, int V, int MODE, int NH>
 __global__ void __launch_bounds__(NT, NH > 1 ? 3 : 1) token_kernel(TokenParams p) {
   using L = TokenSmem<T, K, V, MODE, NH>;

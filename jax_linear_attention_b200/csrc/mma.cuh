@@ -183,7 +183,8 @@ __device__ __forceinline__ void store_acc(T* dst, int ld, int r0, int c0, const 
 }
 
 __device__ __forceinline__ void quad_transpose(uint32_t (&w)[4], int t) {  // w[i] of the quad's lane t <-> w[t] of lane i
-  uint32_t a = __shfl_xor_sync(0xffffffffu, (t & 1) ? w[0] : w[1], 1), b = __shfl_xor_sync(0xffffffffu, (t & 1) ? w[2] : w[3], 1);
+  uint32_t a = __shfl_xor_sync(0xffffffffu, (t & 1) ? w[0] : w[1], 1);
+  uint32_t b = __shfl_xor_sync(0xffffffffu, (t & 1) ? w[2] : w[3], 1);
   if (t & 1) w[0] = a, w[2] = b;
   else w[1] = a, w[3] = b;
   a = __shfl_xor_sync(0xffffffffu, (t & 2) ? w[0] : w[2], 2), b = __shfl_xor_sync(0xffffffffu, (t & 2) ? w[1] : w[3], 2);
@@ -201,11 +202,11 @@ __device__ __forceinline__ void store_row_words(T* dst, uint32_t (&w)[4], int t,
     for (int i = 0; i < 4; ++i) *reinterpret_cast<uint32_t*>(dst + i * 8 + 2 * t) = w[i];
   }
 }
-// An accumulator block (see store_acc) to global memory in 16-byte stores: the four lanes of a quad exchange their words so that each holds eight
-// adjacent columns (4-byte stores write half sectors, and the L2 takes those no faster than whole ones). Mamba-2 walks
-// 173 -> 138 us each, KDA gradient kernels 456 + 241 -> 439 + 236 us. `dst` points at
-// (row 0, column 0) of the block; only the first `rows` of the 16 rows are written
-// (a destination that is not 16-byte aligned takes 4-byte stores).
+// An accumulator block (see store_acc) to global memory in 16-byte stores: the four lanes of a quad exchange their words so
+// that each holds eight adjacent columns (4-byte stores write half sectors, and the L2 takes those no faster than whole
+// ones). Mamba-2 walks 173 -> 138 us each, KDA gradient kernels 456 + 241 -> 439 + 236 us. `dst` points at (row 0,
+// column 0) of the block; only the first `rows` of the 16 rows are written (a destination that is not 16-byte aligned takes
+// 4-byte stores).
 template <typename T, int NT>
 __device__ __forceinline__ void store_acc_wide(T* dst, long ld, const float (&acc)[NT][4], int lane, int rows) {
   static_assert(NT % 4 == 0, "quads of n-tiles");

@@ -328,52 +328,52 @@ __global__ void __launch_bounds__(THREADS, BWD ? (VEC == 4 ? 2 : 1) : (VEC == 4 
         segs[K - 1 + u] = seg_tok(g * UNROLL + u);
       }
       auto tokens = [&](auto same) {
-      constexpr bool kSame = decltype(same)::value;
+        constexpr bool kSame = decltype(same)::value;
 #pragma unroll
-      for (int u = 0; u < UNROLL; ++u) {
-        const int tok = t + u;
-        const bool token = tok < p.T && tok < tend;
-        TokenOut<VEC> o;
-        conv_token<K, VEC, kSame, true>(p, w, bias, rows + u, segs + u, lanes, o);
-        float dnv[VEC];
-        unpack<T, VEC>(dnr[u], dnv);
-        float dot = 0.f;
+        for (int u = 0; u < UNROLL; ++u) {
+          const int tok = t + u;
+          const bool token = tok < p.T && tok < tend;
+          TokenOut<VEC> o;
+          conv_token<K, VEC, kSame, true>(p, w, bias, rows + u, segs + u, lanes, o);
+          float dnv[VEC];
+          unpack<T, VEC>(dnr[u], dnv);
+          float dot = 0.f;
 #pragma unroll
-        for (int c = 0; c < VEC; ++c) dot += dnv[c] * o.y[c];
-        if (p.head_dim > 0) dot = head_sum(dot, lanes);
+          for (int c = 0; c < VEC; ++c) dot += dnv[c] * o.y[c];
+          if (p.head_dim > 0) dot = head_sum(dot, lanes);
 #pragma unroll
-        for (int l = 0; l + 1 < K; ++l) {
+          for (int l = 0; l + 1 < K; ++l) {
 #pragma unroll
-          for (int c = 0; c < VEC; ++c) dp[l][c] = dp[l + 1][c];
-        }
-#pragma unroll
-        for (int c = 0; c < VEC; ++c) {
-          const float dy = p.head_dim > 0 ? o.inv * (dnv[c] - o.y[c] * dot) : dnv[c];
-          const float sg = o.sg[c];
-          dp[K - 1][c] = !token ? 0.f : (p.activation ? dy * sg * (1.f + o.pre[c] * (1.f - sg)) : dy);
-        }
-        if (tok < tb) {  // inside the range: this token's share of the parameter gradients
-          const int sc = segs[u + K - 1];
-#pragma unroll
-          for (int j = 0; j < K; ++j) {
-            if (kSame || j == K - 1 || segs[u + j] == sc) fma_row<VEC>(dwacc[j], dp[K - 1], rows[u + j]);
+            for (int c = 0; c < VEC; ++c) dp[l][c] = dp[l + 1][c];
           }
 #pragma unroll
-          for (int c = 0; c < VEC; ++c) dbacc[c] += dp[K - 1][c];
-        }
-        const int srow = tok - (K - 1);  // its document id is segs[u], that of srow + l is segs[u + l]
-        if (live && srow >= s_lo && srow < tb) {
-          float acc[VEC];
-#pragma unroll
-          for (int c = 0; c < VEC; ++c) acc[c] = 0.f;
-#pragma unroll
-          for (int l = 0; l < K; ++l) {
-            if (l == 0 ? srow >= 0 : kSame || segs[u + l] == segs[u]) fma_row<VEC>(acc, w[K - 1 - l], dp[l]);
+          for (int c = 0; c < VEC; ++c) {
+            const float dy = p.head_dim > 0 ? o.inv * (dnv[c] - o.y[c] * dot) : dnv[c];
+            const float sg = o.sg[c];
+            dp[K - 1][c] = !token ? 0.f : (p.activation ? dy * sg * (1.f + o.pre[c] * (1.f - sg)) : dy);
           }
-          if (srow >= 0) store_row<T, VEC>(dxrow + (long)srow * p.C, acc);
-          else store_row<T, VEC>(static_cast<T*>(p.dstate) + ((long)b * (K - 1) + (K - 1 + srow)) * p.C + col, acc);
+          if (tok < tb) {  // inside the range: this token's share of the parameter gradients
+            const int sc = segs[u + K - 1];
+#pragma unroll
+            for (int j = 0; j < K; ++j) {
+              if (kSame || j == K - 1 || segs[u + j] == sc) fma_row<VEC>(dwacc[j], dp[K - 1], rows[u + j]);
+            }
+#pragma unroll
+            for (int c = 0; c < VEC; ++c) dbacc[c] += dp[K - 1][c];
+          }
+          const int srow = tok - (K - 1);  // its document id is segs[u], that of srow + l is segs[u + l]
+          if (live && srow >= s_lo && srow < tb) {
+            float acc[VEC];
+#pragma unroll
+            for (int c = 0; c < VEC; ++c) acc[c] = 0.f;
+#pragma unroll
+            for (int l = 0; l < K; ++l) {
+              if (l == 0 ? srow >= 0 : kSame || segs[u + l] == segs[u]) fma_row<VEC>(acc, w[K - 1 - l], dp[l]);
+            }
+            if (srow >= 0) store_row<T, VEC>(dxrow + (long)srow * p.C, acc);
+            else store_row<T, VEC>(static_cast<T*>(p.dstate) + ((long)b * (K - 1) + (K - 1 + srow)) * p.C + col, acc);
+          }
         }
-      }
       };
       if (one_document()) tokens(std::true_type{});
       else tokens(std::false_type{});

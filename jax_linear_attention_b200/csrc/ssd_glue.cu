@@ -76,64 +76,64 @@ __global__ void __launch_bounds__(THREADS) ssd_glue_kernel(GlueParams p) {
   const float dh = live && MODE == kLayerBwd ? p.d[h] : 0.f;
   float hacc = 0.f, dacc = 0.f;
   for (long tg = t0; tg < t1; tg += UNROLL) {
-  uint4 xr[UNROLL], orr[UNROLL], yr[UNROLL];
-  float dts[UNROLL], dgs[UNROLL];
+    uint4 xr[UNROLL], orr[UNROLL], yr[UNROLL];
+    float dts[UNROLL], dgs[UNROLL];
 #pragma unroll
-  for (int u = 0; u < UNROLL; ++u) {
-    const bool in = live && tg + u < t1;
-    const long off = (tg + u) * HP + col;
-    const uint4 z = make_uint4(0, 0, 0, 0);
-    xr[u] = in ? *reinterpret_cast<const uint4*>(static_cast<const T*>(p.x) + off) : z;
-    if (MODE != kInputsFwd) orr[u] = in ? *reinterpret_cast<const uint4*>(static_cast<const T*>(p.other) + off) : z;
-    if (MODE != kOutputFwd && MODE != kOutputBwd) dts[u] = in ? p.dt[(tg + u) * p.H + h] : 0.f;
-    if (MODE == kInputsBwd || MODE == kLayerBwd) dgs[u] = in ? p.dg[(tg + u) * p.H + h] : 0.f;
-    if (MODE == kLayerBwd) yr[u] = in ? *reinterpret_cast<const uint4*>(static_cast<const T*>(p.dy) + off) : z;
-  }
-#pragma unroll
-  for (int u = 0; u < UNROLL; ++u) {
-    const long t = tg + u;
-    if (t >= t1) break;
-    const long row = t * p.H + h;
-    const long off = t * HP + col;
-    float xv[8], ov[8] = {}, yv[8] = {}, res[8];
-    unpack8<T>(xr[u], xv);
-    if (MODE != kInputsFwd) unpack8<T>(orr[u], ov);
-    if (MODE == kLayerBwd) unpack8<T>(yr[u], yv);
-    if (MODE == kInputsFwd) {
-      const float dt = dts[u];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) res[i] = xv[i] * dt;
-      if (live && head_lead) p.g[row] = dt * ah;
-    } else if (MODE == kInputsBwd || MODE == kLayerBwd) {
-      const float dt = dts[u];
-      float dot = 0.f;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        // the two-kernel form rounds dv * dt and D * dy to the activation dtype before their sum; here one rounding
-        res[i] = MODE == kLayerBwd ? fmaf(dh, yv[i], ov[i] * dt) : ov[i] * dt;
-        dot += ov[i] * xv[i];
-        if (MODE == kLayerBwd) dacc += yv[i] * xv[i];
-      }
-      const float dg = dgs[u];
-      if (pow2) {
-        dot = group_sum(dot, lanes);
-        if (live && head_lead) p.ddt[row] = dot + dg * ah;
-      } else if (live) {
-        atomicAdd(p.ddt + row, dot + (head_lead ? dg * ah : 0.f));  // ddt zeroed by the launcher in this case
-      }
-      if (head_lead) hacc += dg * dt;
-    } else if (MODE == kOutputFwd) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) res[i] = ov[i] + coef * xv[i];
-    } else {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        res[i] = coef * ov[i];
-        hacc += ov[i] * xv[i];
-      }
+    for (int u = 0; u < UNROLL; ++u) {
+      const bool in = live && tg + u < t1;
+      const long off = (tg + u) * HP + col;
+      const uint4 z = make_uint4(0, 0, 0, 0);
+      xr[u] = in ? *reinterpret_cast<const uint4*>(static_cast<const T*>(p.x) + off) : z;
+      if (MODE != kInputsFwd) orr[u] = in ? *reinterpret_cast<const uint4*>(static_cast<const T*>(p.other) + off) : z;
+      if (MODE != kOutputFwd && MODE != kOutputBwd) dts[u] = in ? p.dt[(tg + u) * p.H + h] : 0.f;
+      if (MODE == kInputsBwd || MODE == kLayerBwd) dgs[u] = in ? p.dg[(tg + u) * p.H + h] : 0.f;
+      if (MODE == kLayerBwd) yr[u] = in ? *reinterpret_cast<const uint4*>(static_cast<const T*>(p.dy) + off) : z;
     }
-    if (live) store8<T>(static_cast<T*>(p.out) + off, res);
-  }
+#pragma unroll
+    for (int u = 0; u < UNROLL; ++u) {
+      const long t = tg + u;
+      if (t >= t1) break;
+      const long row = t * p.H + h;
+      const long off = t * HP + col;
+      float xv[8], ov[8] = {}, yv[8] = {}, res[8];
+      unpack8<T>(xr[u], xv);
+      if (MODE != kInputsFwd) unpack8<T>(orr[u], ov);
+      if (MODE == kLayerBwd) unpack8<T>(yr[u], yv);
+      if (MODE == kInputsFwd) {
+        const float dt = dts[u];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) res[i] = xv[i] * dt;
+        if (live && head_lead) p.g[row] = dt * ah;
+      } else if (MODE == kInputsBwd || MODE == kLayerBwd) {
+        const float dt = dts[u];
+        float dot = 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          // the two-kernel form rounds dv * dt and D * dy to the activation dtype before their sum; here one rounding
+          res[i] = MODE == kLayerBwd ? fmaf(dh, yv[i], ov[i] * dt) : ov[i] * dt;
+          dot += ov[i] * xv[i];
+          if (MODE == kLayerBwd) dacc += yv[i] * xv[i];
+        }
+        const float dg = dgs[u];
+        if (pow2) {
+          dot = group_sum(dot, lanes);
+          if (live && head_lead) p.ddt[row] = dot + dg * ah;
+        } else if (live) {
+          atomicAdd(p.ddt + row, dot + (head_lead ? dg * ah : 0.f));  // ddt zeroed by the launcher in this case
+        }
+        if (head_lead) hacc += dg * dt;
+      } else if (MODE == kOutputFwd) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) res[i] = ov[i] + coef * xv[i];
+      } else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          res[i] = coef * ov[i];
+          hacc += ov[i] * xv[i];
+        }
+      }
+      if (live) store8<T>(static_cast<T*>(p.out) + off, res);
+    }
   }
   if (MODE == kInputsBwd || MODE == kLayerBwd) {
     if (live && head_lead) atomicAdd(p.hsum + h, hacc);
