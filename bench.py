@@ -100,9 +100,18 @@ def kernel_model(K: int, V: int, delta: bool, save: bool) -> dict:
     m["sg_grads_k"] = dict(
         bytes=2 * qk + cc + 2 * st + gates + 256 + qk + ((4 * vv + cc) if delta else vv),
         mac=64 * 64 * K + 64 * K * V + ((64 * 64 * V + 64 * 64 * K + 2 * 64 ** 3 + 2 * 64 * 64 * K + 64 * K * V) if delta else 0))
+    # head sizes with K or V = 64: walks of the state alone, the outputs (and scale P^T dO) for all chunks at once; without
+    # the delta rule the gradient kernel forms dV
+    m["split_fwd"] = dict(bytes=qk + vv + gates + st + (cc + vv if delta else 0),
+                          mac=K * V * 64 * (2 if delta else 1) + (64 * 64 * V if delta else 0))
+    m["split_out"] = dict(bytes=2 * qk + 2 * vv + st + gates, mac=64 * 64 * (K + V) + 64 * K * V)
+    m["split_z"] = dict(bytes=2 * qk + vv + gates + 64 * V * 4, mac=64 * 64 * (K + V))
+    m["split_bwd"] = dict(bytes=qk + vv + gates + st + (qk + cc + 64 * V * 4 + 2 * vv if delta else 0),
+                          mac=64 * K * V * (3 if delta else 1) + (64 * 64 * V if delta else 0))
     m["sg_chunk_grads"] = dict(
-        bytes=2 * qk + 2 * vv + 2 * st + gates + 2 * qk + ((cc + 3 * vv) if delta else 0),
-        mac=64 * 64 * V + 64 * K * V + 64 * 64 * K * 2 + 64 * K * V + ((64 * 64 * V + 64 * K * V + 2 * 64 * 64 * K) if delta else 0))
+        bytes=2 * qk + 2 * vv + 2 * st + gates + 2 * qk + ((cc + 3 * vv) if delta else vv),
+        mac=64 * 64 * V + 64 * K * V + 64 * 64 * K * 2 + 64 * K * V +
+            ((64 * 64 * V + 64 * K * V + 2 * 64 * 64 * K) if delta else 64 * K * V + 64 * 64 * V))
     # KDA (per-channel gates): the gate-folded operands go through HBM between the prologue and the state passes, and
     # the gradients of the folded state-side operands between the two gradient kernels (fp32)
     f32 = 64 * K * 4

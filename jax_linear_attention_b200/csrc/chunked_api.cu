@@ -87,6 +87,11 @@ int chunked_fwd(const jla_problem& p, const jla_fwd_io& io, cudaStream_t stream)
     if (rc != JLA_OK) return rc;
   }
   if (use_tc_kernels(p)) return launch_sg_fwd_tc(c, io, stream);
+  // The split forward keeps the state entering every chunk and Vn for its second kernel, which is memory that a call with
+  // residuals has anyway. A call without them runs the fused walk, whose scratch has no room for either and which the
+  // fixed scratch of jla_linear_attention_fwd_noalloc() relies on; it is the slower of the two (kernels of a forward, us):
+  // 411 against 308 for Mamba-2's B8 T2048 H64 P64 N128, 123 against 45 for B3 T1000 H8 d64 with the delta rule, 2132
+  // against 1334 for B64 T2048 H16 d64, 1048 against 261 for B1 T8192 H16 K64 V128.
   return pl.save ? launch_split_fwd(c, io, stream) : launch_sg_fwd(c, io, stream);
 }
 

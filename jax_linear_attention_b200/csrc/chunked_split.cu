@@ -12,12 +12,12 @@
 // B3 T1000 H8 K = V = 64) and, two CTAs to an SM, 6.9 us a chunk and SM (512 chains of Mamba-2's B8 T2048 H64 P64 N128).
 // Here the walk holds only the chain: three products and three barriers a chunk with the delta rule, one product and one
 // barrier without, on four warps; the value columns of a state are independent, so a call with few chains runs them in
-// blocks of VB. What is read back for the outputs (h, Vn) the backward keeps anyway. Forwards that keep nothing stay on
-// the fused kernel (chunked_fwd.cu), which needs no scratch for h.
+// blocks of VB. What is read back for the outputs (h, Vn) the backward keeps anyway. Forwards that keep nothing run the
+// fused kernel (chunked_fwd.cu): it is slower, but its scratch holds neither (see chunked_api.cu).
 //
-// Measured: the walks of the d = 64 shape 23 + 29 us (fused 109 + 119), of the Mamba-2 shape 139 + 137 us and its outputs
-// 150 us (fused 439 + 436); what bounds them now is the latency of a chunk's loads, barriers and products at one to four
-// CTAs of four warps an SM.
+// Measured: the walks of the d = 64 shape 23 + 29 us (fused, with outputs and scores, 109 + 119), of the Mamba-2 shape 139 +
+// 137 us and its outputs 150 us (fused 439 + 436); what bounds them now is the latency of a chunk's loads, barriers and
+// products at one to four CTAs of four warps an SM.
 //
 // 16-bit operands, fp32 accumulation, the carried state in fp32, Z in fp32. The reverse walk rounds the weighted query
 // fragments (the weighted dO once did); in f16 the weights are lifted to the chunk's largest one first, see state_kernel.
@@ -414,7 +414,7 @@ int run_state(const StateParams& sp, int chains, cudaStream_t s) {
   auto* kern = state_kernel<T, K, VB, DELTA, BWD>;
   constexpr int smem = StateSmem<T, K, VB, DELTA, BWD>::kBytes;
   JLA_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  ProfScope ps(BWD ? kProfSgBwdState : kProfSgFwd, s);
+  ProfScope ps(BWD ? kProfSplitBwd : kProfSplitFwd, s);
   kern<<<chains * (sp.V / VB), NT, smem, s>>>(sp);
   JLA_LAUNCH_OK();
   return JLA_OK;
@@ -433,7 +433,7 @@ int run_tokens_nh(const TokenParams& tp, int nc, cudaStream_t s) {
   auto* kern = token_kernel<T, K, V, MODE, NH>;
   constexpr int smem = TokenSmem<T, K, V, MODE, NH>::kBytes;
   JLA_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  ProfScope ps(kProfSplitTokens, s);
+  ProfScope ps(MODE == kZ ? kProfSplitZ : kProfSplitOut, s);
   kern<<<nc * (tp.H / NH), NT, smem, s>>>(tp);
   JLA_LAUNCH_OK();
   return JLA_OK;

@@ -7,7 +7,8 @@ namespace jla {
 enum {
   kProfTables = 0, kProfGates, kProfL2Norm, kProfKktInv, kProfSgFwd, kProfSgBwdState, kProfSgChunkGrads,
   kProfFinalize, kProfRecFwd, kProfRecBwd, kProfKdaPrep, kProfKdaIntra, kProfKdaFwd, kProfKdaBwdState,
-  kProfKdaChunkGrads, kProfCpCorrection, kProfSgGradsQ, kProfSgGradsK, kProfTokenStep, kProfRecGrads, kProfSplitTokens, kProfKernels
+  kProfKdaChunkGrads, kProfCpCorrection, kProfSgGradsQ, kProfSgGradsK, kProfTokenStep, kProfRecGrads, kProfSplitFwd,
+  kProfSplitOut, kProfSplitZ, kProfSplitBwd, kProfKernels
 };
 
 class ProfScope {

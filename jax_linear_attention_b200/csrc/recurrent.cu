@@ -15,7 +15,7 @@
 // (dS_t = decay (dS_{t+1} + ...), du_t = k_t dS), with its own checkpoints. Everything that needs both, the gradients
 // of q, k and the gates, is then computed for all blocks of TB tokens at once from the two checkpoints of a block.
 //
-// fp32 B1 T512 H4 K = V = 64 forward + backward: 122 + 146 + 17 us of kernels (walk, two walks, block gradients); the
+// fp32 B1 T512 H4 K = V = 64 forward + backward: 120 + 151 + 15 us of kernels (walk, two walks, block gradients); the
 // one-CTA-per-head scan with barriers in every token and the gradient reductions inside the walk took 410 + 2718 us.
 // A token of a walk is 108 instructions of one warp, 240 ns: its chain and the waits of a warp that is alone on its
 // scheduler.
