@@ -283,10 +283,14 @@ def _forward(q, k, v, g, beta, h0, k_read, cfg: dict, needs_grad: bool):
     return o, final, residuals, flags, rows
 
 
+_forward_ad, _functorch_level = torch.autograd.forward_ad, torch._C._functorch.peek_interpreter_stack
+_tracing, _compiling = torch._C._get_tracing_state, torch.compiler.is_compiling
+_PLAIN = frozenset((torch.Tensor, torch.nn.Parameter, type(None)))
+
+
 def _no_transform() -> bool:
     """No forward-mode level, no functorch transform, no tracer."""
-    return (torch.autograd.forward_ad._current_level < 0 and torch._C._functorch.peek_interpreter_stack() is None
-            and torch._C._get_tracing_state() is None and not torch.compiler.is_compiling())
+    return _forward_ad._current_level < 0 and _functorch_level() is None and _tracing() is None and not _compiling()
 
 
 def _bypasses_autograd(tensors) -> bool:
@@ -297,12 +301,12 @@ def _bypasses_autograd(tensors) -> bool:
 
 def nothing_to_differentiate(tensors) -> bool:
     """The same for a layer around the op, which ``no_grad`` calls with parameters: plain tensors or parameters, no
-    transform, and gradients are off or none of them requires one. (A loop: a generator costs a decoding step 0.6 us.)"""
-    grad = torch.is_grad_enabled()
-    for x in tensors:
-        if x is not None:
-            kind = type(x)
-            if (kind is not torch.Tensor and kind is not torch.nn.Parameter) or (grad and x.requires_grad):
+    transform, and gradients are off or none of them requires one. (Written for a decoding step, whose host time it is.)"""
+    if not _PLAIN.issuperset(map(type, tensors)):
+        return False
+    if torch.is_grad_enabled():
+        for x in tensors:
+            if x is not None and x.requires_grad:
                 return False
     return _no_transform()
 
