@@ -83,9 +83,10 @@ def peaks() -> dict:
 
 # Algorithmic work of each kernel per (chunk, head) at K = V = 128, bf16 (bytes it must read + write once; MACs
 # of its products excluding recomputation and the triangular inverse). 1 MAC = 2 FLOP.
-def kernel_model(K: int, V: int, delta: bool, save: bool) -> dict:
+def kernel_model(K: int, V: int, delta: bool, save: bool, group: int = 1) -> dict:
+    """``group``: value heads that share a key head, hence the tiles of q and k (and of their gradients)."""
     e = 2
-    qk, vv, st, cc = 64 * K * e, 64 * V * e, K * V * e, 64 * 64 * e
+    qk, vv, st, cc = 64 * K * e / group, 64 * V * e, K * V * e, 64 * 64 * e
     gates = 128 * 4 + 64
     m = {}
     if delta:
@@ -611,7 +612,8 @@ def main() -> None:
         if V > 128 and V % 128 == 0:  # wide value heads run as V / 128 heads of 128 channels: count those
             H, V = H * (V // 128), 128
         units = (tokens // CHUNK) * H  # (chunk, head) pairs per launch
-        model = kernel_model(K, V, delta=args.workload != "ssd", save=True)
+        model = kernel_model(K, V, delta=args.workload != "ssd", save=True,
+                             group=H // (case["q"].shape[2] if "q" in case else case["B"].shape[2]))
         roof = None
         step_traffic = 0.0
         step_traffic_known = bool(prof)
@@ -626,7 +628,7 @@ def main() -> None:
             top = max(prof, key=lambda n: prof[n]["total_ms"])
             per_launch_ms = prof[top]["total_ms"] / prof[top]["launches"]
             if top in model:
-                by = model[top]["bytes"] * units
+                by = round(model[top]["bytes"] * units)
                 fl = 2 * model[top]["mac"] * units
                 t_hbm = by / (pk["hbm_gbs"] * 1e9)
                 t_tc = fl / (pk["bf16_tflops"] * 1e12)
