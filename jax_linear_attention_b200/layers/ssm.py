@@ -73,14 +73,14 @@ def _step(x, dt, a, b, c, d, segment_ids, initial_state, output_final_state, chu
     batch, _, heads, width = x.shape
     groups, n = b.shape[2:]
     options = dict(initial_state=initial_state, segment_ids=segment_ids, chunk_size=chunk_size, precision=precision)
-    b = ops.cuda.cast(b, c.dtype)
+    cast, dev, f32 = ops.cuda.cast, x.device, torch.float32
+    b = cast(b, c.dtype, dev)
     if (batch == 0 or c.dtype != x.dtype or n not in (64, 128, 256) or width % 64 or precision == "chunked"
             or (d is not None and d.shape != (heads,))
             or ops.cuda._reason("simple_gla", c, b, x, (dt,), options) is not None):
         return None
-    dev, f32 = x.device, torch.float32
-    c, b, x = (ops.cuda.cast(t, c.dtype, dev) for t in (c, b, x))
-    dt, a, d, initial_state = (ops.cuda.cast(t, f32, dev) for t in (dt, a, d, initial_state))
+    c, x, dt, a, d = cast(c, c.dtype, dev), cast(x, c.dtype, dev), cast(dt, f32, dev), cast(a, f32, dev), cast(d, f32, dev)
+    initial_state = cast(initial_state, f32, dev)
     p = ops.cuda._problem("simple_gla", x.dtype, batch, 1, heads, groups, n, width, 0, 1.0, 0, precision,
                           c.data_ptr(), b.data_ptr(), x.data_ptr(), None, None,
                           None if initial_state is None else initial_state.data_ptr())
