@@ -15,7 +15,7 @@
 // (dS_t = decay (dS_{t+1} + ...), du_t = k_t dS), with its own checkpoints. Everything that needs both, the gradients
 // of q, k and the gates, is then computed for all blocks of TB tokens at once from the two checkpoints of a block.
 //
-// fp32 B1 T512 H4 K = V = 64 forward + backward: 120 + 151 + 15 us of kernels (walk, two walks, block gradients); the
+// fp32 B1 T512 H4 K = V = 64 forward + backward: 119 + 145 + 16 us of kernels (walk, two walks, block gradients); the
 // one-CTA-per-head scan with barriers in every token and the gradient reductions inside the walk took 410 + 2718 us.
 // A token of a walk is 108 instructions of one warp, 240 ns: its chain and the waits of a warp that is alone on its
 // scheduler.
@@ -536,10 +536,10 @@ __global__ void __launch_bounds__(GT) block_grads_kernel(RecParams p) {
   {  // u_j . do_t and u_j . dr_t, one pair (j, t) a thread
     const int j = tid / TB, t = tid % TB;
     float at = 0.f, ct = 0.f;
-    for (int x0 = 0; x0 < V; x0 += VT) {  // (sums of short sums: the rounding of a long chain would show in dg)
+    for (int x0 = 0; x0 < V; x0 += VT / 2) {  // (sums of short sums: the rounding of a long chain would show in dq and dg)
       float a[4] = {}, c[4] = {};
-#pragma unroll 4
-      for (int x = x0; x < min(V, x0 + VT); x += 4) {
+#pragma unroll
+      for (int x = x0; x < min(V, x0 + VT / 2); x += 4) {
         const float4 u = *reinterpret_cast<const float4*>(s.u + j * s.vs + x);
         const float4 d = *reinterpret_cast<const float4*>(s.d + t * s.vs + x);
         const float4 r = *reinterpret_cast<const float4*>(s.r + t * s.vs + x);
@@ -572,25 +572,30 @@ __global__ void __launch_bounds__(GT) block_grads_kernel(RecParams p) {
       }
       __syncthreads();
       const int xe = min(VT, V - x0);
-      float td[4] = {}, tr[4] = {}, tu[4] = {}, tn = 0.f;
-      for (int x = 0; x < xe; x += 4) {
-        const float4 a = *reinterpret_cast<const float4*>(s.ts + cl * VTS + x);
-        const float4 g = *reinterpret_cast<const float4*>(s.te + cl * VTS + x);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int at = (tq + i) * s.vs + x0 + x;
-          const float4 d = *reinterpret_cast<const float4*>(s.d + at);
-          const float4 r = *reinterpret_cast<const float4*>(s.r + at);
-          const float4 u = *reinterpret_cast<const float4*>(s.u + at);
-          td[i] += (a.x * d.x + a.y * d.y) + (a.z * d.z + a.w * d.w);
-          tr[i] += (a.x * r.x + a.y * r.y) + (a.z * r.z + a.w * r.w);
-          tu[i] += (g.x * u.x + g.y * u.y) + (g.z * u.z + g.w * u.w);
+      for (int xh = 0; xh < VT; xh += VT / 2) {  // (short sums here too)
+        float td[4] = {}, tr[4] = {}, tu[4] = {}, tn = 0.f;
+#pragma unroll
+        for (int x = xh; x < xh + VT / 2; x += 4) {
+          if (x >= xe) break;
+          const float4 a = *reinterpret_cast<const float4*>(s.ts + cl * VTS + x);
+          const float4 g = *reinterpret_cast<const float4*>(s.te + cl * VTS + x);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int at = (tq + i) * s.vs + x0 + x;
+            const float4 d = *reinterpret_cast<const float4*>(s.d + at);
+            const float4 r = *reinterpret_cast<const float4*>(s.r + at);
+            const float4 u = *reinterpret_cast<const float4*>(s.u + at);
+            td[i] += (a.x * d.x + a.y * d.y) + (a.z * d.z + a.w * d.w);
+            tr[i] += (a.x * r.x + a.y * r.y) + (a.z * r.z + a.w * r.w);
+            tu[i] += (g.x * u.x + g.y * u.y) + (g.z * u.z + g.w * u.w);
+          }
+          if ((x / 4 & 3) == tg) tn += (g.x * a.x + g.y * a.y) + (g.z * a.z + g.w * a.w);
         }
-        if ((x / 4 & 3) == tg) tn += (g.x * a.x + g.y * a.y) + (g.z * a.z + g.w * a.w);
-      }
 #pragma unroll
-      for (int i = 0; i < 4; ++i) ad[i] += td[i], ar[i] += tr[i], au[i] += tu[i];
-      en += tn;
+        for (int i = 0; i < 4; ++i) ad[i] += td[i], ar[i] += tr[i], au[i] += tu[i];
+        en += tn;
+      }
     }
     // ---- the in-block terms of this thread's channel and four tokens; the products of decays grow one token at a time
     const int c = c0 + cl;
@@ -598,6 +603,7 @@ __global__ void __launch_bounds__(GT) block_grads_kernel(RecParams p) {
     // Of dg: A_ji of this thread's tokens i passes through the tokens j + 1 .. i. For the tokens up to tq that is all four i,
     // whose sum is kept per j; behind tq, token tq + m takes those of i >= m.
     float pairs[TB - 1], behind[4] = {}, qs[4], krs[4];
+    float odd_q[4], odd_r[4];  // terms join dq and dkr two at a time: half the roundings of the growing sums
 #pragma unroll
     for (int i = 0; i < 4; ++i) qs[i] = p.scale * s.q[(tq + i) * s.K + c], krs[i] = s.kr[(tq + i) * s.K + c];
     auto add_pairs = [&](const float (&a)[4]) {
@@ -616,14 +622,16 @@ __global__ void __launch_bounds__(GT) block_grads_kernel(RecParams p) {
       float a[4] = {};
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
+        float xq = 0.f, xr = 0.f;
         if (tq + i >= j) {
           w[i] = cut ? 0.f : w[i] * e;
-          if (w[i] != 0.f) {
-            const float xq = w[i] * kp * xs[i], xr = w[i] * kp * ys[i];
-            dq[i] += xq, dkr[i] += xr;
+          if (j > 0 && w[i] != 0.f) {
+            xq = w[i] * kp * xs[i], xr = w[i] * kp * ys[i];
             a[i] = qs[i] * xq + krs[i] * xr;
           }
         }
+        if (j & 1) odd_q[i] = xq, odd_r[i] = xr;
+        else dq[i] += odd_q[i] + xq, dkr[i] += odd_r[i] + xr;
       }
       if (j > 0) {  // (a predecessor among this thread's own tokens does not pass through those up to itself)
         const int own = j - 1 - tq;
